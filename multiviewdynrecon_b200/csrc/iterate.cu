@@ -433,8 +433,6 @@ __device__ inline int term_rows(const InstDesc& I, const TermOffsets& off, const
 
 // ------------------------------------------ diagonal blocks, Jt r, M^-1 ----
 
-__device__ constexpr int upper_index(int i, int j) { return i * 6 - (i * (i - 1)) / 2 + (j - i); }
-
 // DenseGaussian<6>::Inverse with partial pivoting (DenseGaussian.h:55-125)
 __device__ inline void gauss_jordan6(const float* Din, float* out) {
     float m[36];
@@ -466,23 +464,24 @@ __device__ inline void gauss_jordan6(const float* Din, float* out) {
 // 6x6 Cholesky in double; packed lower triangle L[i(i+1)/2 + j], j <= i, with
 // the RECIPROCALS of the diagonal stored on the diagonal so that the solves
 // applied every PCG iteration only multiply
-template <class T> __device__ inline void cholesky6(const T* A, double* L) {
+// (a column per instantiation, so that every index is a constant and the factor
+// stays in registers)
+template <int j, class T> __device__ inline void cholesky6_column(const T (&A)[36], double (&L)[21]) {
+    double s = A[6 * j + j];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
-        double s = A[6 * j + j];
+    for (int k = 0; k < j; ++k) s -= L[j * (j + 1) / 2 + k] * L[j * (j + 1) / 2 + k];
+    const double inv = 1.0 / sqrt(s);
+    L[j * (j + 1) / 2 + j] = inv;
 #pragma unroll
-        for (int k = 0; k < j; ++k) s -= L[j * (j + 1) / 2 + k] * L[j * (j + 1) / 2 + k];
-        const double inv = 1.0 / sqrt(s);
-        L[j * (j + 1) / 2 + j] = inv;
+    for (int i = j + 1; i < 6; ++i) {
+        double t = A[6 * i + j];
 #pragma unroll
-        for (int i = j + 1; i < 6; ++i) {
-            double t = A[6 * i + j];
-#pragma unroll
-            for (int k = 0; k < j; ++k) t -= L[i * (i + 1) / 2 + k] * L[j * (j + 1) / 2 + k];
-            L[i * (i + 1) / 2 + j] = t * inv;
-        }
+        for (int k = 0; k < j; ++k) t -= L[i * (i + 1) / 2 + k] * L[j * (j + 1) / 2 + k];
+        L[i * (i + 1) / 2 + j] = t * inv;
     }
+    if constexpr (j < 5) cholesky6_column<j + 1>(A, L);
 }
+template <class T> __device__ inline void cholesky6(const T (&A)[36], double (&L)[21]) { cholesky6_column<0>(A, L); }
 
 __device__ inline void cholesky6_solve(const double* L, const double* b, double* x) {
     double y[6];
@@ -517,6 +516,10 @@ template <> struct BlockStore<false> {
     __device__ static V* ptr(const InstDesc& I) { return I.bsr; }
 };
 
+template <class V> struct Pair;
+template <> struct Pair<double> { using type = double2; };
+template <> struct Pair<float> { using type = float2; };
+
 // ------------------------------------------------- JtJ block helpers -----
 // Twist Jacobian row of a point-to-point or smooth residual at point p
 // (geometry_icp_jacobian.cuh:91-120, 323-343): f_c(p) = [row c of [p]x^T ; e_c].
@@ -526,26 +529,9 @@ template <class T> __device__ inline void twist_rows(T px, T py, T pz, T f[3][6]
     f[2][0] = py;  f[2][1] = -px; f[2][2] = 0;   f[2][3] = 0; f[2][4] = 0; f[2][5] = 1;
 }
 
-// (sum_c f_c(p) f_c(q)^T)(r, k) for the twist rows above; with r and k known
-// at compile time this folds to at most three products
-template <class T> __device__ inline T twist_rows_product(const T p[3], const T q[3], int r, int k) {
-    // f_c(p)[r] for r < 3: the rows of [p]x^T
-    auto sk = [](const T v[3], int c, int rr) -> T {
-        if (c == 0) return rr == 0 ? (T)0 : (rr == 1 ? v[2] : -v[1]);
-        if (c == 1) return rr == 0 ? -v[2] : (rr == 1 ? (T)0 : v[0]);
-        return rr == 0 ? v[1] : (rr == 1 ? -v[0] : (T)0);
-    };
-    if (r < 3 && k < 3) return sk(p, 0, r) * sk(q, 0, k) + sk(p, 1, r) * sk(q, 1, k) + sk(p, 2, r) * sk(q, 2, k);
-    if (r < 3) return sk(p, k - 3, r);
-    if (k < 3) return sk(q, r - 3, k);
-    return r == k ? (T)1 : (T)0;
-}
-
 // upper-triangle index of a symmetric 6x6 block (r <= k)
 __device__ constexpr int sym_idx(int r, int k) { return r * 6 - (r * (r - 1)) / 2 + (k - r); }
 
-// S += sg g^T on the upper triangle (sg is a multiple of g, so the product is
-// symmetric)
 // S += (c g) g^T on the upper triangle, (c g_r) formed once per row r
 template <class Acc>
 __device__ inline void add_scaled_outer(Acc S[21], Acc c, const Acc g[6]) {
@@ -557,12 +543,18 @@ __device__ inline void add_scaled_outer(Acc S[21], Acc c, const Acc g[6]) {
     }
 }
 
-template <class Acc>
-__device__ inline void add_sym_outer(Acc S[21], const Acc sg[6], const Acc g[6]) {
-#pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-        for (int k = r; k < 6; ++k) S[sym_idx(r, k)] += sg[r] * g[k];
+// Asynchronous copies into shared memory (through the L2 only), in groups per
+// thread
+__device__ inline void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ inline void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ inline void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// index of a pixel term's record in term_jr (kInvalid: not a pixel term)
+__device__ inline uint32_t pixel_record_index(const TermOffsets& off, uint32_t t) {
+    if (t < off.o[0]) return t;
+    return t >= off.o[1] && t < off.o[2] ? off.o[0] + (t - off.o[1]) : kInvalid;
 }
 
 // ---------------------------------------------------- diagonal blocks ----
@@ -570,321 +562,658 @@ __device__ inline void add_sym_outer(Acc S[21], const Acc sg[6], const Acc g[6])
 // D_i = sum_t lambda_t^2 w_ti^2 sum_c g_c g_c^T (21 upper-triangle sums) and
 // b_i = -sum_t lambda_t^2 w_ti sum_c g_c r_c (6 sums) in registers; a fixed
 // reduce-scatter (five halving exchanges) then leaves each of 27 lanes with
-// one warp total, so the result does not depend on scheduling. computeBlockDiagonalPreconditionerKernel and
-// computeJtResidualWithIndexKernel (PreconditionerBlocked.cu:18-399,
-// JtDotResidualIndexed.cu:18-382) compute the same sums. A CTA takes
-// kDiagNodes nodes; their damped blocks wait in shared memory and one warp
-// then factors them, a node per lane (Cholesky in double for mixed precision,
-// the Gauss-Jordan inverse of BlockDiagonalPreconditionerInverse.cu:7-60 in
-// float).
-constexpr uint32_t kDiagNodes = 32;
+// one warp total, so the result does not depend on scheduling.
+// computeBlockDiagonalPreconditionerKernel and computeJtResidualWithIndexKernel
+// (PreconditionerBlocked.cu:18-399, JtDotResidualIndexed.cu:18-382) compute the
+// same sums. The 54 accumulator registers leave room for 16 warps per SM, so
+// the latency of the record gathers is covered by asynchronous copies into the
+// lanes' own slots of shared memory, kDiagStages - 1 terms ahead of the sums; and
+// a warp takes one node, where eight in turn left most of a frame's SMs idle.
+// Measured alone, us: 500-node frame 18 (was 85), 4096-node frame 25 (69),
+// 32,768-node frame 260 (323).
+constexpr uint32_t kDiagWarps = 4;
+constexpr uint32_t kDiagStages = 4;
 
-// 4 CTAs per SM (128 registers, no spills): with the term loads software-
-// pipelined, fewer but spill-free warps win (measured against 5 CTAs)
-template <bool MIXED>
-__global__ void __launch_bounds__(128, 4) diag_rhs_kernel(const InstDesc* insts, mvdr_penalty lam) {
+template <bool MIXED, bool DENS>
+__global__ void __launch_bounds__(32 * kDiagWarps, 4) diag_rhs_kernel(const InstDesc* insts, mvdr_penalty lam) {
     using Acc = typename std::conditional<MIXED, double, float>::type;
-    __shared__ Acc s_blocks[kDiagNodes][21];
+    __shared__ float4 s_rec[kDiagWarps][kDiagStages][2][32];
+    __shared__ float4 s_dens[DENS ? kDiagWarps : 1][kDiagStages][2][32];
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
-    if (C->node2term_entries > I.cap_k1 || C->half_pairs > I.cap_pairs) return;
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint32_t node = blockIdx.x * kDiagWarps + warp;
+    if (node >= I.N || C->node2term_entries > I.cap_k1 || C->half_pairs > I.cap_pairs) return;
     TermOffsets off;
     off.load(C);
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const Acc l2_fg = (Acc)(lam.foreground * lam.foreground), l2_smooth = (Acc)(lam.smooth * lam.smooth);
     const Acc l2_feat = (Acc)(lam.feature * lam.feature), l2_cross = (Acc)(lam.cross_view * lam.cross_view);
     // the density channel of the dense pixels (0 when the term is off or its
     // weight is 0 in this iteration's phase)
-    const bool dens_on = I.use_density && lam.density != 0.f;
+    const bool dens_on = DENS && I.use_density && lam.density != 0.f;
     const Acc l2_dens = (Acc)(lam.density * lam.density);
     // the upper-triangle entry (orr, okk) of D whose total this lane receives
     uint32_t orr = 0, okk = 0;
     for (uint32_t r = 0, q = 0; r < 6; ++r)
         for (uint32_t k = r; k < 6; ++k, ++q)
             if (q == lane) { orr = r; okk = k; }
-    for (uint32_t base = blockIdx.x * kDiagNodes; base < I.N; base += gridDim.x * kDiagNodes) {
-        for (uint32_t j = warp; j < kDiagNodes && base + j < I.N; j += nwarps) {
-            const uint32_t node = base + j;
-            const uint32_t b0 = I.n2t_offset[node], b1 = I.n2t_offset[node + 1];
-            Acc S[21], R[6];
+    const uint32_t b0 = I.n2t_offset[node], b1 = I.n2t_offset[node + 1];
+    Acc S[21], R[6];
 #pragma unroll
-            for (int q = 0; q < 21; ++q) S[q] = 0;
+    for (int q = 0; q < 21; ++q) S[q] = 0;
 #pragma unroll
-            for (int q = 0; q < 6; ++q) R[q] = 0;
-            // software pipeline over the lane's terms: the term id two steps
-            // ahead and the pixel-term record and weight one step ahead are in
-            // flight while the current term is summed
-            uint32_t t1 = b0 + lane < b1 ? I.n2t_index[b0 + lane] : kInvalid;
-            uint32_t t2 = b0 + lane + 32 < b1 ? I.n2t_index[b0 + lane + 32] : kInvalid;
-            float4 pa = make_float4(0.f, 0.f, 0.f, 0.f), pb = pa;
-            float pw = 0.f;
-            auto fetch_pixel_term = [&](uint32_t t, uint32_t pp) {
-                uint32_t k;
-                const TermType ty = off.typed(t, k);
-                if (ty == kDense || ty == kForeground) {
-                    const uint32_t idx = ty == kDense ? k : off.o[0] + k;
-                    pa = I.term_jr[2 * (size_t)idx];
-                    pb = I.term_jr[2 * (size_t)idx + 1];
-                    pw = I.n2t_w[pp];
-                }
-            };
-            if (b0 + lane < b1) fetch_pixel_term(t1, b0 + lane);
-            for (uint32_t p = b0 + lane; p < b1; p += 32) {
-                const uint32_t t = t1;
-                const float4 a = pa, b = pb;
-                const float wf = pw;
-                t1 = t2;
-                if (p + 64 < b1) t2 = I.n2t_index[p + 64];
-                if (p + 32 < b1) fetch_pixel_term(t1, p + 32);
-                uint32_t k;
-                const TermType ty = off.typed(t, k);
-                if (ty == kDense || ty == kForeground) {
-                    const Acc w = (Acc)wf;
-                    if (__float_as_uint(b.w) != kInvalid) {  // an invalid term has J = 0, r = 0
-                        const Acc l2 = ty == kDense ? (Acc)1 : l2_fg;
-                        const Acc g[6] = {(Acc)a.x, (Acc)a.y, (Acc)a.z, (Acc)a.w, (Acc)b.x, (Acc)b.y};
-                        const Acc sw = l2 * w * w, rw = -l2 * w * (Acc)b.z;
-#pragma unroll
-                        for (int q = 0; q < 6; ++q) R[q] += rw * g[q];
-                        add_scaled_outer(S, sw, g);
-                    }
-                    if (ty == kDense && dens_on) {
-                        float4 da, db;
-                        load_record32(I.density_jr + 2 * (size_t)k, da, db);
-                        if (__float_as_uint(db.w) != kInvalid) {
-                            const Acc g[6] = {(Acc)da.x, (Acc)da.y, (Acc)da.z, (Acc)da.w, (Acc)db.x, (Acc)db.y};
-                            const Acc sw = l2_dens * w * w, rw = -l2_dens * w * (Acc)db.z;
-#pragma unroll
-                            for (int q = 0; q < 6; ++q) R[q] += rw * g[q];
-                            add_scaled_outer(S, sw, g);
-                        }
-                    }
-                } else if (ty == kSmooth) {
-                    // computeSmoothTermJacobian (geometry_icp_jacobian.cuh:323-343):
-                    // J_i,c = f_c(T_i x_j), J_j,c = -f_c(T_j x_j)
-                    const float4 a = I.smooth[3 * (size_t)k], b = I.smooth[3 * (size_t)k + 1];
-                    if (b.z == 0.f) continue;
-                    const float4 rr = I.smooth[3 * (size_t)k + 2];
-                    const bool is_i = node == I.graph[k].x;
-                    const float4 pt = is_i ? a : make_float4(a.w, b.x, b.y, 0.f);
-                    Acc fr[3][6];
-                    twist_rows<Acc>((Acc)pt.x, (Acc)pt.y, (Acc)pt.z, fr);
-                    const Acc rc[3] = {(Acc)rr.x, (Acc)rr.y, (Acc)rr.z};
-                    const Acc sgn = is_i ? (Acc)1 : (Acc)-1;
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const Acc rw = -l2_smooth * sgn * rc[c];
-#pragma unroll
-                        for (int q = 0; q < 6; ++q) R[q] += rw * fr[c][q];
-                        add_scaled_outer(S, l2_smooth, fr[c]);
-                    }
-                } else if (ty == kFeature || ty == kCross) {
-                    const bool f = ty == kFeature;
-                    const float4 wv = I.warped[2 * (size_t)(f ? k : I.Tp + k)];
-                    const float4 raw = I.warped[2 * (size_t)(f ? k : I.Tp + k) + 1];
-                    const Acc l2 = f ? l2_feat : l2_cross;
-                    const Acc w = (Acc)I.n2t_w[p];
-                    Acc fr[3][6];
-                    twist_rows<Acc>((Acc)wv.x, (Acc)wv.y, (Acc)wv.z, fr);
-                    const float rv[3] = {raw.x, raw.y, raw.z};
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const Acc hw = (Acc)huber_weight(rv[c]);
-                        const Acc rw = -l2 * hw * (Acc)rv[c];
-                        Acc g[6];
-#pragma unroll
-                        for (int q = 0; q < 6; ++q) {
-                            g[q] = w * hw * fr[c][q];
-                            R[q] += rw * g[q];
-                        }
-                        add_scaled_outer(S, l2, g);
-                    }
-                }
-            }
-            // fixed-order reduce-scatter: five halving steps leave lane q with
-            // the warp total of value q (q < 21: D entry q, 21 + k: b_k)
-            Acc v[32];
-#pragma unroll
-            for (int q = 0; q < 21; ++q) v[q] = S[q];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) v[21 + q] = R[q];
-#pragma unroll
-            for (int q = 27; q < 32; ++q) v[q] = 0;
-#pragma unroll
-            for (int dist = 16; dist > 0; dist >>= 1) {
-                const bool upper = (lane & (uint32_t)dist) != 0;
-#pragma unroll
-                for (int i = 0; i < dist; ++i) {
-                    const Acc keep = upper ? v[i + dist] : v[i];
-                    const Acc send = upper ? v[i] : v[i + dist];
-                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, dist);
-                }
-            }
-            const Acc tot = v[0];
-            const size_t blk = 36 * (size_t)(I.half_offset[node] + node);
-            typename BlockStore<MIXED>::V* store = BlockStore<MIXED>::ptr(I);
-            if (lane < 21) {
-                const Acc d = tot + (orr == okk ? (Acc)1e-2f : (Acc)0);  // damping
-                I.diag[36 * (size_t)node + 6 * orr + okk] = (float)d;
-                I.diag[36 * (size_t)node + 6 * okk + orr] = (float)d;
-                store[blk + blk_idx(orr, okk)] = d;
-                store[blk + blk_idx(okk, orr)] = d;
-                s_blocks[j][lane] = d;
-            } else if (lane < 27) {
-                PcgVec<MIXED>::jtr(I)[6 * (size_t)node + lane - 21] = tot;
+    for (int q = 0; q < 6; ++q) R[q] = 0;
+    // pipeline over the lane's terms: the records of the next
+    // kDiagStages - 1 terms are being copied to shared memory, and the
+    // term id of the one after them is in flight
+    uint32_t ring_t[kDiagStages];
+    float ring_w[kDiagStages];
+    auto request = [&](uint32_t t, uint32_t p, uint32_t slot) {
+        const uint32_t rec = p < b1 ? pixel_record_index(off, t) : kInvalid;
+        if (rec != kInvalid) {
+            copy_async16(&s_rec[warp][slot][0][lane], I.term_jr + 2 * (size_t)rec);
+            copy_async16(&s_rec[warp][slot][1][lane], I.term_jr + 2 * (size_t)rec + 1);
+            if (dens_on && t < off.o[0]) {
+                copy_async16(&s_dens[DENS ? warp : 0][slot][0][lane], I.density_jr + 2 * (size_t)t);
+                copy_async16(&s_dens[DENS ? warp : 0][slot][1][lane], I.density_jr + 2 * (size_t)t + 1);
             }
         }
-        __syncthreads();
-        if (warp == 0 && base + lane < I.N) {
-            const uint32_t node = base + lane;
-            Acc D[36];
+        copy_commit();
+    };
+    uint32_t t_next;
+    float w_next;
+    auto load_ids = [&](uint32_t p) {
+        t_next = p < b1 ? I.n2t_index[p] : kInvalid;
+        w_next = p < b1 ? I.n2t_w[p] : 0.f;
+    };
 #pragma unroll
-            for (int r = 0; r < 6; ++r)
+    for (uint32_t q = 0; q < kDiagStages - 1; ++q) {
+        load_ids(b0 + lane + 32 * q);
+        ring_t[q] = t_next;
+        ring_w[q] = w_next;
+    }
 #pragma unroll
-                for (int k2 = 0; k2 < 6; ++k2) D[6 * r + k2] = s_blocks[lane][r <= k2 ? sym_idx(r, k2) : sym_idx(k2, r)];
-            if constexpr (MIXED) {
-                double L[21];
-                cholesky6(D, L);
+    for (uint32_t q = 0; q < kDiagStages - 1; ++q) request(ring_t[q], b0 + lane + 32 * q, q);
+    load_ids(b0 + lane + 32 * (kDiagStages - 1));
+    for (uint32_t p = b0 + lane, slot = kDiagStages - 1; p < b1; p += 32) {
+        slot = (slot + 1) % kDiagStages;
+        const uint32_t t = ring_t[0];
+        const float wf = ring_w[0];
 #pragma unroll
-                for (int i = 0; i < 21; ++i) I.chol[21 * (size_t)node + i] = L[i];
-            } else {
-                float Df[36], Mi[36];
+        for (uint32_t q = 0; q + 2 < kDiagStages; ++q) {
+            ring_t[q] = ring_t[q + 1];
+            ring_w[q] = ring_w[q + 1];
+        }
+        ring_t[kDiagStages - 2] = t_next;
+        ring_w[kDiagStages - 2] = w_next;
+        request(t_next, p + 32 * (kDiagStages - 1), (slot + kDiagStages - 1) % kDiagStages);
+        load_ids(p + 32 * kDiagStages);
+        copy_wait<kDiagStages - 1>();
+        const float4 a = s_rec[warp][slot][0][lane], b = s_rec[warp][slot][1][lane];
+        uint32_t k;
+        const TermType ty = off.typed(t, k);
+        if (ty == kDense || ty == kForeground) {
+            const Acc w = (Acc)wf;
+            if (__float_as_uint(b.w) != kInvalid) {  // an invalid term has J = 0, r = 0
+                const Acc l2 = ty == kDense ? (Acc)1 : l2_fg;
+                const Acc g[6] = {(Acc)a.x, (Acc)a.y, (Acc)a.z, (Acc)a.w, (Acc)b.x, (Acc)b.y};
+                const Acc sw = l2 * w * w, rw = -l2 * w * (Acc)b.z;
 #pragma unroll
-                for (int i = 0; i < 36; ++i) Df[i] = (float)D[i];
-                gauss_jordan6(Df, Mi);
+                for (int q = 0; q < 6; ++q) R[q] += rw * g[q];
+                add_scaled_outer(S, sw, g);
+            }
+            if (ty == kDense && dens_on) {
+                const float4 da = s_dens[DENS ? warp : 0][slot][0][lane], db = s_dens[DENS ? warp : 0][slot][1][lane];
+                if (__float_as_uint(db.w) != kInvalid) {
+                    const Acc g[6] = {(Acc)da.x, (Acc)da.y, (Acc)da.z, (Acc)da.w, (Acc)db.x, (Acc)db.y};
+                    const Acc sw = l2_dens * w * w, rw = -l2_dens * w * (Acc)db.z;
 #pragma unroll
-                for (int i = 0; i < 36; ++i) I.minv[36 * (size_t)node + i] = Mi[i];
+                    for (int q = 0; q < 6; ++q) R[q] += rw * g[q];
+                    add_scaled_outer(S, sw, g);
+                }
+            }
+        } else if (ty == kSmooth) {
+            // computeSmoothTermJacobian (geometry_icp_jacobian.cuh:323-343):
+            // J_i,c = f_c(T_i x_j), J_j,c = -f_c(T_j x_j)
+            const float4 a = I.smooth[3 * (size_t)k], b = I.smooth[3 * (size_t)k + 1];
+            if (b.z == 0.f) continue;
+            const float4 rr = I.smooth[3 * (size_t)k + 2];
+            const bool is_i = node == I.graph[k].x;
+            const float4 pt = is_i ? a : make_float4(a.w, b.x, b.y, 0.f);
+            Acc fr[3][6];
+            twist_rows<Acc>((Acc)pt.x, (Acc)pt.y, (Acc)pt.z, fr);
+            const Acc rc[3] = {(Acc)rr.x, (Acc)rr.y, (Acc)rr.z};
+            const Acc sgn = is_i ? (Acc)1 : (Acc)-1;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const Acc rw = -l2_smooth * sgn * rc[c];
+#pragma unroll
+                for (int q = 0; q < 6; ++q) R[q] += rw * fr[c][q];
+                add_scaled_outer(S, l2_smooth, fr[c]);
+            }
+        } else if (ty == kFeature || ty == kCross) {
+            const bool f = ty == kFeature;
+            const float4 wv = I.warped[2 * (size_t)(f ? k : I.Tp + k)];
+            const float4 raw = I.warped[2 * (size_t)(f ? k : I.Tp + k) + 1];
+            const Acc l2 = f ? l2_feat : l2_cross;
+            const Acc w = (Acc)wf;
+            Acc fr[3][6];
+            twist_rows<Acc>((Acc)wv.x, (Acc)wv.y, (Acc)wv.z, fr);
+            const float rv[3] = {raw.x, raw.y, raw.z};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const Acc hw = (Acc)huber_weight(rv[c]);
+                const Acc rw = -l2 * hw * (Acc)rv[c];
+                Acc g[6];
+#pragma unroll
+                for (int q = 0; q < 6; ++q) {
+                    g[q] = w * hw * fr[c][q];
+                    R[q] += rw * g[q];
+                }
+                add_scaled_outer(S, l2, g);
             }
         }
-        __syncthreads();
+    }
+    // fixed-order reduce-scatter: five halving steps leave lane q with
+    // the warp total of value q (q < 21: D entry q, 21 + k: b_k)
+    Acc v[32];
+#pragma unroll
+    for (int q = 0; q < 21; ++q) v[q] = S[q];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) v[21 + q] = R[q];
+#pragma unroll
+    for (int q = 27; q < 32; ++q) v[q] = 0;
+#pragma unroll
+    for (int dist = 16; dist > 0; dist >>= 1) {
+        const bool upper = (lane & (uint32_t)dist) != 0;
+#pragma unroll
+        for (int i = 0; i < dist; ++i) {
+            const Acc keep = upper ? v[i + dist] : v[i];
+            const Acc send = upper ? v[i] : v[i + dist];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, dist);
+        }
+    }
+    const Acc tot = v[0];
+    const size_t blk = 36 * (size_t)(I.half_offset[node] + node);
+    typename BlockStore<MIXED>::V* store = BlockStore<MIXED>::ptr(I);
+    if (lane < 21) {
+        const Acc d = tot + (orr == okk ? (Acc)1e-2f : (Acc)0);  // damping
+        I.diag[36 * (size_t)node + 6 * orr + okk] = (float)d;
+        I.diag[36 * (size_t)node + 6 * okk + orr] = (float)d;
+        store[blk + blk_idx(orr, okk)] = d;
+        store[blk + blk_idx(okk, orr)] = d;
+    } else if (lane < 27) {
+        PcgVec<MIXED>::jtr(I)[6 * (size_t)node + lane - 21] = tot;
     }
 }
 
-// --------------------------------------------------- off-diagonal blocks --
-// One thread per unordered pair (i < j), accumulating in registers. Every
-// term type but smooth contributes w_i w_j lambda^2 sum_c g_c g_c^T (dense and
-// foreground: one channel g = J; feature and cross: three Huber-weighted twist
-// rows), a symmetric product, so the thread keeps the 21 upper-triangle sums
-// only. A pair has at most two smooth terms (its graph edges i->j and j->i);
-// their asymmetric contribution -lambda_s^2 sum_c f_c(p_i) f_c(p_j)^T is added
-// when the block is written. computeJtJNonDiagonalBlockKernel and
-// computeSmoothJtJBlock (JtJMaterializer.cu:20-528, jtj_block_jacobian.cuh:8-65)
-// compute the same sums; only the upper block (i, j) is stored, (j, i) is read
-// as its transpose.
+// The block preconditioner from the damped diagonal blocks, a thread per node:
+// the Cholesky factor in double (mixed precision) or the Gauss-Jordan inverse
+// of BlockDiagonalPreconditionerInverse.cu:7-60 in float. A launch of its own,
+// so that no warp of the assembly waits with its registers for one lane's
+// square roots; it runs beside the off-diagonal blocks.
 template <bool MIXED>
-__global__ void __launch_bounds__(128, 4) offdiag_kernel(const InstDesc* insts, mvdr_penalty lam) {
-    using Acc = typename std::conditional<MIXED, double, float>::type;
+__global__ void __launch_bounds__(64) factor_kernel(const InstDesc* insts) {
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
-    if (C->node2term_entries > I.cap_k1 || C->half_pairs > I.cap_pairs || C->nodepair_entries > I.cap_k2) return;
-    TermOffsets off;
-    off.load(C);
-    const uint32_t P = C->half_pairs;
-    const Acc l2_fg = (Acc)(lam.foreground * lam.foreground);
-    const Acc l2_feat = (Acc)(lam.feature * lam.feature), l2_cross = (Acc)(lam.cross_view * lam.cross_view);
-    const bool dens_on = I.use_density && lam.density != 0.f;
-    const Acc l2_dens = (Acc)(lam.density * lam.density);
-    // pairs grouped by entry count, so the lanes of a warp loop equally long
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
-        const uint32_t h = I.pair_order[i];
-        const uint32_t ni = I.half_key[h] / I.enc;
-        const uint2 rg = I.half_range[h];
-        Acc S[21];
+    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
+    if (node >= I.N || C->node2term_entries > I.cap_k1 || C->half_pairs > I.cap_pairs) return;
+    using V = typename BlockStore<MIXED>::V;
+    using V2 = typename Pair<V>::type;
+    const V2* blk = reinterpret_cast<const V2*>(BlockStore<MIXED>::ptr(I) + 36 * (size_t)(I.half_offset[node] + node));
+    V D[36];
 #pragma unroll
-        for (int q = 0; q < 21; ++q) S[q] = 0;
-        uint32_t smooth_k[2] = {kInvalid, kInvalid};
-        // software pipeline over the pair's entries: the term id two entries
-        // ahead and the pixel-term record one entry ahead are in flight while
-        // the current entry is summed
-        uint32_t t_next = rg.x < rg.y ? I.np_index[rg.x] : 0u;
-        uint32_t t_next2 = rg.x + 1 < rg.y ? I.np_index[rg.x + 1] : 0u;
-        float4 pa = make_float4(0.f, 0.f, 0.f, 0.f), pb = pa;
-        float2 pw = make_float2(0.f, 0.f);
-        auto fetch_pixel_term = [&](uint32_t t, uint32_t p) {
-            uint32_t k;
-            const TermType ty = off.typed(t, k);
-            if (ty == kDense || ty == kForeground) {
-                const uint32_t idx = ty == kDense ? k : off.o[0] + k;
-                load_record32(I.term_jr + 2 * (size_t)idx, pa, pb);
-                pw = I.np_w[p];
-            }
-        };
-        if (rg.x < rg.y) fetch_pixel_term(t_next, rg.x);
-        for (uint32_t p = rg.x; p < rg.y; ++p) {
-            const uint32_t t = t_next;
-            const float4 a = pa, b = pb;
-            const float2 wij = pw;
-            t_next = t_next2;
-            if (p + 2 < rg.y) t_next2 = I.np_index[p + 2];
-            if (p + 1 < rg.y) fetch_pixel_term(t_next, p + 1);
-            uint32_t k;
-            const TermType ty = off.typed(t, k);
-            if (ty == kDense || ty == kForeground) {
-                const Acc wij2 = (Acc)wij.x * (Acc)wij.y;
-                if (__float_as_uint(b.w) != kInvalid) {  // an invalid term has J = 0
-                    const Acc s = ty == kForeground ? wij2 * l2_fg : wij2;
-                    const Acc g[6] = {(Acc)a.x, (Acc)a.y, (Acc)a.z, (Acc)a.w, (Acc)b.x, (Acc)b.y};
-                    add_scaled_outer(S, s, g);
-                }
-                if (ty == kDense && dens_on) {
+    for (int e = 0; e < 18; ++e) {  // pair e: elements (r, 2c) and (r, 2c + 1) (blk_idx)
+        const V2 v = blk[e];
+        D[6 * (e % 6) + 2 * (e / 6)] = v.x;
+        D[6 * (e % 6) + 2 * (e / 6) + 1] = v.y;
+    }
+    if constexpr (MIXED) {
+        double L[21];
+        cholesky6(D, L);
+#pragma unroll
+        for (int i = 0; i < 21; ++i) I.chol[21 * (size_t)node + i] = L[i];
+    } else {
+        float Mi[36];
+        gauss_jordan6(D, Mi);
+#pragma unroll
+        for (int i = 0; i < 36; ++i) I.minv[36 * (size_t)node + i] = Mi[i];
+    }
+}
+
+// row c of a point-to-point term (3 Huber-weighted twist rows) or of a smooth
+// term (hw = 1) at point p
+template <class Acc>
+__device__ inline void twist_row(Acc px, Acc py, Acc pz, uint32_t c, Acc (&g)[6]) {
+    Acc f[3][6];
+    twist_rows<Acc>(px, py, pz, f);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) g[q] = c == 0 ? f[0][q] : (c == 1 ? f[1][q] : f[2][q]);
+}
+
+// --------------------------------------------------- off-diagonal blocks --
+// Every term type but smooth contributes w_i w_j lambda^2 sum_c g_c g_c^T to the
+// block of a pair (i < j) (dense and foreground: one channel g = J; feature and
+// cross: three Huber-weighted twist rows), a symmetric product, so the 21
+// upper-triangle sums suffice. A pair has at most two smooth terms (its graph
+// edges i->j and j->i); their asymmetric contribution
+// -lambda_s^2 sum_c f_c(p_i) f_c(p_j)^T is added when the block is written.
+// computeJtJNonDiagonalBlockKernel and computeSmoothJtJBlock
+// (JtJMaterializer.cu:20-528, jtj_block_jacobian.cuh:8-65) compute the same
+// sums; only the upper block (i, j) is stored, (j, i) is read as its transpose.
+//
+// Each element is one running sum over the pair's entries in list order (the
+// increments of late iterations move with the last bits of these sums), so the
+// launch lasts as long as its longest chain: the longest pairs have several
+// hundred entries, the median one 30 to 60. The pairs come longest first
+// (pair_order); the longest of each window are taken 16 lanes per pair, the rest
+// a thread per pair, in two launches side by side. Both walk the list in the
+// same order with the same operations and give the same bits.
+// The longer of the two launches, us, against one thread per pair with one
+// record in flight: 500-node frame 62 (was 262), 2048-node FP32 frame 63 (308),
+// 4096-node frame 70 (197), 32,768-node frame 317 (663; half of its record
+// gathers miss the L2).
+
+// the pair's smooth terms' points (p_i, p_j), has[m]: the term is valid
+template <class Acc>
+__device__ inline void smooth_points(const InstDesc& I, uint32_t ni, const uint32_t (&smooth_k)[2], Acc (&pi)[2][3],
+                                     Acc (&pj)[2][3], bool (&has)[2]) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        has[m] = false;
+        if (smooth_k[m] == kInvalid) continue;
+        const uint32_t k = smooth_k[m];
+        const float4 a = I.smooth[3 * (size_t)k], b = I.smooth[3 * (size_t)k + 1];
+        if (b.z == 0.f) continue;
+        const bool is_i = ni == I.graph[k].x;
+        const float4 qi = is_i ? a : make_float4(a.w, b.x, b.y, 0.f);
+        const float4 qj = is_i ? make_float4(a.w, b.x, b.y, 0.f) : a;
+        pi[m][0] = (Acc)qi.x; pi[m][1] = (Acc)qi.y; pi[m][2] = (Acc)qi.z;
+        pj[m][0] = (Acc)qj.x; pj[m][1] = (Acc)qj.y; pj[m][2] = (Acc)qj.z;
+        has[m] = true;
+    }
+}
+
+// a * b + c in one rounding; a * b
+__device__ inline double fused(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ inline float fused(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ inline double rounded_product(double a, double b) { return __dmul_rn(a, b); }
+__device__ inline float rounded_product(float a, float b) { return __fmul_rn(a, b); }
+
+// (sum_c f_c(p) f_c(q)^T)(r, k) for the twist rows f_c(p) = [row c of [p]x^T ; e_c]
+template <class T> __device__ inline T twist_product(const T (&p)[3], const T (&q)[3], uint32_t r, uint32_t k) {
+    auto at = [](const T (&v)[3], uint32_t i) { return i == 0 ? v[0] : (i == 1 ? v[1] : v[2]); };
+    // element i of row c of [v]x^T, i != c
+    auto sk = [&](const T (&v)[3], uint32_t c, uint32_t i) {
+        const T x = at(v, 3 - c - i);
+        return (i + 3 - c) % 3 == 1 ? x : -x;
+    };
+    if (r < 3 && k < 3) {
+        if (r != k) return -(at(p, k) * at(q, r));
+        const uint32_t u = r == 1 ? 0 : 1, v = r == 2 ? 0 : 2;  // the two other axes
+        return fused(at(p, u), at(q, u), rounded_product(at(p, v), at(q, v)));
+    }
+    if (r < 3) return k - 3 == r ? (T)0 : sk(p, k - 3, r);
+    if (k < 3) return r - 3 == k ? (T)0 : sk(q, r - 3, k);
+    return r == k ? (T)1 : (T)0;
+}
+
+// v + l (sum_c f_c(p) f_c(q)^T)(r, k). A smooth term's J_i,c = +-f_c(p_i),
+// J_j,c = -+f_c(p_j), so its product carries a minus
+// (geometry_icp_jacobian.cuh:323-343). Every rounding is written out, so that
+// both forms of the kernel give the same bits.
+template <class T>
+__device__ inline T add_twist_product(T v, T l, const T (&p)[3], const T (&q)[3], uint32_t r, uint32_t k) {
+    if (r < 3 && k >= 3) return v + rounded_product(l, twist_product<T>(p, q, r, k));
+    return fused(l, twist_product<T>(p, q, r, k), v);
+}
+
+constexpr uint32_t kPairGroups = kPairChunk / 16;  // groups of 16 lanes per CTA
+// One thread per pair: the records of the next G entries are in flight and the
+// ids of the G after them on the way. Dense entries, nearly all, take the short
+// path; each slot's next load is issued as soon as its record is converted.
+template <class Acc>
+__device__ inline void pair_by_thread(const InstDesc& I, const TermOffsets& off, const mvdr_penalty& lam, uint32_t h,
+                                      Acc* blocks) {
+    constexpr uint32_t G = sizeof(Acc) == 8 ? 2 : 3;  // (the records in flight fill the registers)
+    const uint32_t Td = off.o[0];
+    const bool dens_on = I.use_density && lam.density != 0.f;
+    const float4* jr = I.term_jr;
+    const uint32_t* index = I.np_index;
+    const double* scale = I.np_scale;
+    const uint2 rg = I.half_range[h];
+    Acc S[21];
+#pragma unroll
+    for (int q = 0; q < 21; ++q) S[q] = 0;
+    uint32_t smooth_k[2] = {kInvalid, kInvalid};
+    // (ids past the end are kInvalid: no dense term, never loaded or summed)
+    uint32_t t0[G], t1[G];
+    float4 ra[G], rb[G];
+    double sc[G];
+    // the 32-byte record of a term (none for a smooth term)
+    auto fetch = [&](uint32_t t, float4& x, float4& y) {
+        const float4* src = jr + 2 * (size_t)t;
+        if (t >= Td) {
+            if (t < off.o[1] || t == kInvalid) return;
+            if (t < off.o[2]) src = jr + 2 * (size_t)(Td + (t - off.o[1]));
+            else src = I.warped + 2 * (size_t)(t < off.o[3] ? t - off.o[2] : I.Tp + (t - off.o[3]));
+        }
+        load_record32(src, x, y);
+    };
+    auto ids = [&](uint32_t p, uint32_t (&t)[G]) {
+#pragma unroll
+        for (uint32_t q = 0; q < G; ++q) t[q] = p + q < rg.y ? index[p + q] : kInvalid;
+    };
+    ids(rg.x, t0);
+    ids(rg.x + G, t1);
+#pragma unroll
+    for (uint32_t q = 0; q < G; ++q) {
+        fetch(t0[q], ra[q], rb[q]);
+        if (t0[q] != kInvalid) sc[q] = scale[rg.x + q];
+    }
+    for (uint32_t p = rg.x; p < rg.y; p += G) {
+        uint32_t tn[G];
+        ids(p + 2 * G, tn);
+#pragma unroll
+        for (uint32_t q = 0; q < G; ++q) {
+            const uint32_t t = t0[q];
+            const Acc s = (Acc)sc[q];
+            if (t < Td) {
+                const float4 a = ra[q], b = rb[q];
+                const Acc g[6] = {(Acc)a.x, (Acc)a.y, (Acc)a.z, (Acc)a.w, (Acc)b.x, (Acc)b.y};
+                // the slot's next record, as soon as this one is converted
+                fetch(t1[q], ra[q], rb[q]);
+                if (t1[q] != kInvalid) sc[q] = scale[p + G + q];
+                add_scaled_outer(S, s, g);  // (an invalid term has J = 0)
+                if (dens_on) {
                     float4 da, db;
-                    load_record32(I.density_jr + 2 * (size_t)k, da, db);
-                    if (__float_as_uint(db.w) != kInvalid) {
-                        const Acc g[6] = {(Acc)da.x, (Acc)da.y, (Acc)da.z, (Acc)da.w, (Acc)db.x, (Acc)db.y};
-                        add_scaled_outer(S, wij2 * l2_dens, g);
+                    load_record32(I.density_jr + 2 * (size_t)t, da, db);
+                    const Acc gd[6] = {(Acc)da.x, (Acc)da.y, (Acc)da.z, (Acc)da.w, (Acc)db.x, (Acc)db.y};
+                    add_scaled_outer(S, s * (Acc)(lam.density * lam.density), gd);
+                }
+            } else if (t != kInvalid) {
+                const float4 a = ra[q], b = rb[q];
+                fetch(t1[q], ra[q], rb[q]);
+                if (t1[q] != kInvalid) sc[q] = scale[p + G + q];
+                if (t < off.o[1]) {
+                    if (smooth_k[0] == kInvalid) smooth_k[0] = t - Td;
+                    else smooth_k[1] = t - Td;
+                } else if (t < off.o[2]) {
+                    const Acc g[6] = {(Acc)a.x, (Acc)a.y, (Acc)a.z, (Acc)a.w, (Acc)b.x, (Acc)b.y};
+                    add_scaled_outer(S, s * (Acc)(lam.foreground * lam.foreground), g);
+                } else {  // a = the warped point, b = the raw residual
+                    const float l = t < off.o[3] ? lam.feature : lam.cross_view;
+                    const Acc sl = s * (Acc)(l * l);
+#pragma unroll 1
+                    for (uint32_t c = 0; c < 3; ++c) {
+                        const Acc hw = (Acc)huber_weight(c == 0 ? b.x : (c == 1 ? b.y : b.z));
+                        Acc g[6];
+                        twist_row<Acc>((Acc)a.x, (Acc)a.y, (Acc)a.z, c, g);
+#pragma unroll
+                        for (int e = 0; e < 6; ++e) g[e] *= hw;
+                        add_scaled_outer(S, sl, g);
                     }
                 }
-            } else if (ty == kSmooth) {
+            }
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < G; ++q) {
+            t0[q] = t1[q];
+            t1[q] = tn[q];
+        }
+    }
+    const uint32_t ni = I.half_key[h] / I.enc;
+    Acc pi[2][3], pj[2][3];
+    bool has[2];
+    smooth_points<Acc>(I, ni, smooth_k, pi, pj, has);
+    const Acc l2_smooth = -(Acc)(lam.smooth * lam.smooth);
+    Acc* out = blocks + 36 * (size_t)(h + ni + 1);
+#pragma unroll
+    for (int r = 0; r < 6; ++r)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            Acc v = S[r <= k ? sym_idx(r, k) : sym_idx(k, r)];
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+                if (has[m]) v = add_twist_product<Acc>(v, l2_smooth, pi[m], pj[m], r, k);
+            out[blk_idx(r, k)] = v;
+        }
+}
+
+// 16 lanes per pair, two pairs per warp. The group loads 16 consecutive entries
+// at once, a lane each, and stages each entry's rows s g and g in shared memory;
+// lane u then owns two adjacent elements of the upper triangle and adds the
+// staged entries in order. The next 16 entries' loads are in flight meanwhile.
+// Its bound is the shared-memory reads (three instructions for 4 elements of 2
+// pairs), more per entry than the thread form costs, but the chain per entry is a
+// fifth of it.
+struct BlockUnit {
+    uint32_t r, m;  // elements (r, 2m) and (r, 2m + 1)
+    bool on;
+    // the units with an element on or above the diagonal: rows 0, 1: m = 0-2,
+    // rows 2, 3: m = 1, 2, rows 4, 5: m = 2
+    __device__ inline explicit BlockUnit(uint32_t gl) {
+        on = gl < 12;
+        if (gl < 6) { r = gl / 3; m = gl % 3; }
+        else if (gl < 10) { r = 2 + ((gl - 6) >> 1); m = 1 + ((gl - 6) & 1); }
+        else { r = 4 + (gl & 1); m = 2; }
+    }
+};
+// staged values per entry: s g (6), two of padding, g (6); the stride keeps the
+// 16-byte stores of neighbouring lanes in different banks
+constexpr uint32_t kRowStride = 14, kRowG = 8;
+
+// v[0..1] += the unit's products over staged entries [0, n); with `st2` the two
+// stages alternate entry by entry
+template <bool TWO, class Acc>
+__device__ inline void add_staged(const Acc* st, const Acc* st2, const BlockUnit& u, uint32_t n, Acc (&v)[2]) {
+    using A2 = typename Pair<Acc>::type;
+    const uint32_t og = kRowG + 2 * u.m;
+#pragma unroll 4
+    for (uint32_t e = 0; e < n; ++e) {
+        const Acc s = st[kRowStride * e + u.r];
+        const A2 w = *reinterpret_cast<const A2*>(st + kRowStride * e + og);
+        v[0] = fused(s, w.x, v[0]);
+        v[1] = fused(s, w.y, v[1]);
+        if constexpr (TWO) {
+            const Acc s2 = st2[kRowStride * e + u.r];
+            const A2 w2 = *reinterpret_cast<const A2*>(st2 + kRowStride * e + og);
+            v[0] = fused(s2, w2.x, v[0]);
+            v[1] = fused(s2, w2.y, v[1]);
+        }
+    }
+}
+template <class Acc> __device__ inline void stage_row(Acc* o, Acc s, const Acc (&g)[6]) {
+    using A2 = typename Pair<Acc>::type;
+    A2* o2 = reinterpret_cast<A2*>(o);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        A2 t;
+        t.x = s * g[2 * i];
+        t.y = s * g[2 * i + 1];
+        o2[i] = t;
+        t.x = g[2 * i];
+        t.y = g[2 * i + 1];
+        o2[kRowG / 2 + i] = t;
+    }
+}
+template <class Acc> __device__ inline void stage_zero(Acc* o) {
+    const Acc z[6] = {0, 0, 0, 0, 0, 0};
+    stage_row<Acc>(o, (Acc)0, z);
+}
+// the larger of the two groups' values (loops are warp-uniform)
+__device__ inline uint32_t warp_pair_max(uint32_t v) { return max(v, __shfl_xor_sync(0xffffffffu, v, 16)); }
+
+template <class Acc, bool DENS>
+__device__ inline void pair_by_group(const InstDesc& I, const TermOffsets& off, const mvdr_penalty& lam, uint32_t h,
+                                     Acc* st, Acc* st2, Acc* blocks) {
+    using A2 = typename Pair<Acc>::type;
+    const uint32_t gl = threadIdx.x & 15u, shift = threadIdx.x & 16u;
+    const BlockUnit u(gl);
+    const Acc l2_fg = (Acc)(lam.foreground * lam.foreground);
+    const Acc l2_feat = (Acc)(lam.feature * lam.feature), l2_cross = (Acc)(lam.cross_view * lam.cross_view);
+    const Acc l2_smooth = -(Acc)(lam.smooth * lam.smooth);
+    const bool dens_on = DENS && I.use_density && lam.density != 0.f;
+    const Acc l2_dens = (Acc)(lam.density * lam.density);
+    const bool own = h != kInvalid;
+    const uint2 rg = own ? I.half_range[h] : make_uint2(0u, 0u);
+    const uint32_t len = rg.y - rg.x;
+    Acc v[2] = {0, 0};
+    uint32_t smooth_k[2] = {kInvalid, kInvalid}, tail = rg.y;
+    auto term_at = [&](uint32_t p) { return p < rg.y ? I.np_index[p] : kInvalid; };
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    double w = 0.0;
+    auto fetch = [&](uint32_t t, uint32_t p) {
+        const uint32_t rec = pixel_record_index(off, t);
+        if (rec != kInvalid) {
+            load_record32(I.term_jr + 2 * (size_t)rec, a, b);
+            w = I.np_scale[p];
+        }
+    };
+    uint32_t t1 = term_at(rg.x + gl), t2 = term_at(rg.x + 16 + gl);
+    fetch(t1, rg.x + gl);
+    const uint32_t steps = warp_pair_max((len + 15) / 16);
+    for (uint32_t q = 0; q < steps; ++q) {
+        const uint32_t p = rg.x + 16 * q + gl, t = t1;
+        const bool dense = t < off.o[0], fg = t >= off.o[1] && t < off.o[2];
+        Acc* o = st + kRowStride * gl;
+        const Acc wij = (Acc)w;
+        if (dense || fg) {
+            const Acc g[6] = {(Acc)a.x, (Acc)a.y, (Acc)a.z, (Acc)a.w, (Acc)b.x, (Acc)b.y};
+            stage_row<Acc>(o, fg ? wij * l2_fg : wij, g);  // (an invalid term has J = 0)
+        } else {
+            stage_zero<Acc>(o);
+        }
+        if (dens_on) {
+            Acc* o2 = st2 + kRowStride * gl;
+            if (dense) {
+                float4 da, db;
+                load_record32(I.density_jr + 2 * (size_t)t, da, db);
+                const Acc g[6] = {(Acc)da.x, (Acc)da.y, (Acc)da.z, (Acc)da.w, (Acc)db.x, (Acc)db.y};
+                stage_row<Acc>(o2, wij * l2_dens, g);
+            } else {
+                stage_zero<Acc>(o2);
+            }
+        }
+        t1 = t2;
+        t2 = term_at(p + 32);
+        fetch(t1, p + 16);
+        // the pair's smooth terms, and where its point-to-point tail begins
+        uint32_t ms = (__ballot_sync(0xffffffffu, t >= off.o[0] && t < off.o[1]) >> shift) & 0xFFFFu;
+        const uint32_t mt = (__ballot_sync(0xffffffffu, t >= off.o[2] && t != kInvalid) >> shift) & 0xFFFFu;
+        while (__any_sync(0xffffffffu, ms != 0)) {
+            const uint32_t src = ms ? __ffs(ms) - 1 : 0u;
+            const uint32_t k = __shfl_sync(0xffffffffu, t, shift + src) - off.o[0];
+            if (ms) {
                 if (smooth_k[0] == kInvalid) smooth_k[0] = k;
                 else smooth_k[1] = k;
-            } else if (ty == kFeature || ty == kCross) {
-                const bool f = ty == kFeature;
-                const float4 wv = I.warped[2 * (size_t)(f ? k : I.Tp + k)];
-                const float4 rw = I.warped[2 * (size_t)(f ? k : I.Tp + k) + 1];
-                const float2 wp = I.np_w[p];
-                const Acc s = (Acc)wp.x * (Acc)wp.y * (f ? l2_feat : l2_cross);
-                const float hw[3] = {huber_weight(rw.x), huber_weight(rw.y), huber_weight(rw.z)};
-                Acc fr[3][6];
-                twist_rows<Acc>((Acc)wv.x, (Acc)wv.y, (Acc)wv.z, fr);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    Acc g[6];
-#pragma unroll
-                    for (int q = 0; q < 6; ++q) g[q] = (Acc)hw[c] * fr[c][q];
-                    add_scaled_outer(S, s, g);
-                }
+                ms &= ms - 1;
             }
         }
-        // smooth terms: J_i,c = +-f_c(p_i), J_j,c = -+f_c(p_j), so their
-        // product carries a minus (geometry_icp_jacobian.cuh:323-343); the
-        // elements of sum_c f_c(p_i) f_c(p_j)^T come from the two points
-        Acc pi[2][3], pj[2][3];
-        bool has[2] = {false, false};
+        if (mt && tail == rg.y) tail = rg.x + 16 * q + __ffs(mt) - 1;
+        const uint32_t n = warp_pair_max(16 * q < len ? min(16u, len - 16 * q) : 0u);
+        __syncwarp();
+        if (dens_on) add_staged<DENS, Acc>(st, st2, u, n, v);
+        else add_staged<false, Acc>(st, st, u, n, v);
+        __syncwarp();
+    }
+    // point-to-point terms, five by three rows per step
+    const uint32_t rest = warp_pair_max((rg.y - tail + 4) / 5);
+    for (uint32_t q = 0; q < rest; ++q) {
+        const uint32_t p = tail + 5 * q + gl / 3, c = gl % 3;
+        Acc* o = st + kRowStride * gl;
+        if (gl < 15 && p < rg.y) {
+            uint32_t k;
+            const bool f = off.typed(I.np_index[p], k) == kFeature;
+            const float4 wv = I.warped[2 * (size_t)(f ? k : I.Tp + k)];
+            const float4 rw = I.warped[2 * (size_t)(f ? k : I.Tp + k) + 1];
+            const Acc s = (Acc)I.np_scale[p] * (f ? l2_feat : l2_cross);
+            const Acc hw = (Acc)huber_weight(c == 0 ? rw.x : (c == 1 ? rw.y : rw.z));
+            Acc g[6];
+            twist_row<Acc>((Acc)wv.x, (Acc)wv.y, (Acc)wv.z, c, g);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            if (smooth_k[m] == kInvalid) continue;
-            const uint32_t k = smooth_k[m];
-            const float4 a = I.smooth[3 * (size_t)k], b = I.smooth[3 * (size_t)k + 1];
-            if (b.z == 0.f) continue;
-            const bool is_i = ni == I.graph[k].x;
-            const float4 qi = is_i ? a : make_float4(a.w, b.x, b.y, 0.f);
-            const float4 qj = is_i ? make_float4(a.w, b.x, b.y, 0.f) : a;
-            pi[m][0] = (Acc)qi.x; pi[m][1] = (Acc)qi.y; pi[m][2] = (Acc)qi.z;
-            pj[m][0] = (Acc)qj.x; pj[m][1] = (Acc)qj.y; pj[m][2] = (Acc)qj.z;
-            has[m] = true;
+            for (int i = 0; i < 6; ++i) g[i] *= hw;
+            stage_row<Acc>(o, s, g);
+        } else {
+            stage_zero<Acc>(o);
         }
-        const Acc l2_smooth = -(Acc)(lam.smooth * lam.smooth);
-        typename BlockStore<MIXED>::V* out = BlockStore<MIXED>::ptr(I) + 36 * (size_t)(h + ni + 1);
+        __syncwarp();
+        add_staged<false, Acc>(st, st, u, 15u, v);
+        __syncwarp();
+    }
+    // the block in shared memory, then out in element pairs (blk_idx) with
+    // the smooth terms added
+    if (u.on) {
 #pragma unroll
-        for (int r = 0; r < 6; ++r)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                Acc v = S[r <= k ? sym_idx(r, k) : sym_idx(k, r)];
-#pragma unroll
-                for (int m = 0; m < 2; ++m)
-                    if (has[m]) v += l2_smooth * twist_rows_product<Acc>(pi[m], pj[m], r, k);
-                out[blk_idx(r, k)] = v;
+        for (uint32_t q = 0; q < 2; ++q) {
+            const uint32_t k = 2 * u.m + q;
+            if (u.r <= k) {
+                st[6 * u.r + k] = v[q];
+                st[6 * k + u.r] = v[q];
             }
+        }
+    }
+    const uint32_t ni = own ? I.half_key[h] / I.enc : 0u;
+    Acc pi[2][3], pj[2][3];
+    bool has[2];
+    smooth_points<Acc>(I, ni, smooth_k, pi, pj, has);
+    __syncwarp();
+    if (own) {
+        A2* out = reinterpret_cast<A2*>(blocks + 36 * (size_t)(h + ni + 1));
+        for (uint32_t e = gl; e < 18; e += 16) {  // pair e: elements (r, 2c) and (r, 2c + 1)
+            const uint32_t r = e % 6, c = e / 6;
+            Acc x[2] = {st[6 * r + 2 * c], st[6 * r + 2 * c + 1]};
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                if (!has[m]) continue;
+                x[0] = add_twist_product<Acc>(x[0], l2_smooth, pi[m], pj[m], r, 2 * c);
+                x[1] = add_twist_product<Acc>(x[1], l2_smooth, pi[m], pj[m], r, 2 * c + 1);
+            }
+            A2 o;
+            o.x = x[0];
+            o.y = x[1];
+            out[e] = o;
+        }
+    }
+    __syncwarp();
+}
+
+// true when the pair lists are complete (the host call reports what is not)
+__device__ inline bool pair_lists_complete(const InstDesc& I) {
+    const DeviceCounts* C = I.counts;
+    return C->node2term_entries <= I.cap_k1 && C->half_pairs <= I.cap_pairs && C->nodepair_entries <= I.cap_k2;
+}
+
+// the first `share` pairs of every window (pair_order), kPairGroups per CTA step
+template <bool MIXED, bool DENS>
+__global__ void __launch_bounds__(kPairChunk, 7) offdiag_group_kernel(const InstDesc* insts, mvdr_penalty lam, uint32_t share) {
+    using Acc = typename BlockStore<MIXED>::V;
+    __shared__ __align__(16) Acc s_stage[DENS ? 2 : 1][kPairGroups][16 * kRowStride];
+    const InstDesc& I = insts[blockIdx.y];
+    if (!pair_lists_complete(I)) return;
+    TermOffsets off;
+    off.load(I.counts);
+    const uint32_t windows = pair_slots(I.counts->half_pairs) / kPairWindow, group = threadIdx.x >> 4;
+    for (uint32_t item = blockIdx.x; item < windows * (share / kPairGroups); item += gridDim.x) {
+        // (pairs of about equal length in a warp's two groups)
+        const uint32_t pos = (item % windows) * kPairChunk + (item / windows) * kPairGroups + group;
+        pair_by_group<Acc, DENS>(I, off, lam, I.pair_order[pos], s_stage[0][group], s_stage[DENS ? 1 : 0][group],
+                                 BlockStore<MIXED>::ptr(I));
+    }
+}
+
+// the other pairs
+template <bool MIXED>
+__global__ void __launch_bounds__(kPairChunk, 4) offdiag_thread_kernel(const InstDesc* insts, mvdr_penalty lam, uint32_t share) {
+    const InstDesc& I = insts[blockIdx.y];
+    if (!pair_lists_complete(I)) return;
+    TermOffsets off;
+    off.load(I.counts);
+    const uint32_t slots = pair_slots(I.counts->half_pairs), first = slots / kPairWindow * kPairChunk;
+    for (uint32_t pos = blockIdx.x * kPairChunk + threadIdx.x; pos < slots; pos += gridDim.x * kPairChunk) {
+        if (pos < first && threadIdx.x < share) continue;
+        const uint32_t h = I.pair_order[pos];
+        if (h != kInvalid) pair_by_thread<typename BlockStore<MIXED>::V>(I, off, lam, h, BlockStore<MIXED>::ptr(I));
     }
 }
 
@@ -1222,10 +1551,6 @@ __global__ void __launch_bounds__(256) pcg_direction_kernel(const InstDesc* inst
 // tile, so it is usually still in L2.
 const SpmvShape kSpmvShapes[kNumSpmvShapes] = {{16, 2, 0}, {8, 2, 0},  {16, 1, 0}, {32, 1, 0}, {16, 3, 0}, {8, 4, 0},
                                                 {32, 2, 0}, {16, 1, 1}, {32, 1, 1}, {8, 2, 1},  {16, 2, 1}, {4, 4, 1}};
-
-template <class V> struct Pair;
-template <> struct Pair<double> { using type = double2; };
-template <> struct Pair<float> { using type = float2; };
 
 // the SpMV operand: this iteration's direction
 template <bool MIXED> __device__ inline const typename BlockStore<MIXED>::V* direction(const InstDesc& I, int parity) {
@@ -2238,44 +2563,81 @@ static void launch_apply_pair(const LaunchCfg& lc, InstDesc* d, const float* x, 
     }
 }
 
+// the diagonal blocks with Jt r, then the preconditioner
+template <bool MIXED>
+static void launch_diag(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
+    const dim3 grid = grid2((lc.max_nodes + kDiagWarps - 1) / kDiagWarps, lc.B);
+    if (lc.use_density) MVDR_LAUNCH((diag_rhs_kernel<MIXED, true>), grid, 32 * kDiagWarps, 0, st, d, lam);
+    else MVDR_LAUNCH((diag_rhs_kernel<MIXED, false>), grid, 32 * kDiagWarps, 0, st, d, lam);
+    MVDR_LAUNCH(factor_kernel<MIXED>, grid2((lc.max_nodes + 63) / 64, lc.B), 64, 0, st, d);
+}
+static void launch_diag(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
+    if (lc.precision == MVDR_PRECISION_MIXED) launch_diag<true>(lc, d, lam, st);
+    else launch_diag<false>(lc, d, lam, st);
+}
+
+// Pairs of each window taken by group. By group a pair's chain is five times
+// shorter but its entries cost seven times the instructions: an eighth of the
+// pairs while the launch is bound by its chains; few where it has other work to
+// fill the GPU meanwhile. Whole solves, ms, with 128 / 32 / 8 of 1024: 500-node
+// frame 1.49 / 1.63 / -, 4096-node frame 2.38 / 2.52 / -, 32,768-node frame 16.2 /
+// 15.8 / -, 16 x 4096 nodes in two lanes 10.74 / 10.53 / 10.31.
+static uint32_t group_share(const LaunchCfg& lc) {
+    if ((uint64_t)lc.B * lc.max_nodes < 16384) return kPairChunk;
+    return lc.B < 4 ? 32 : 8;
+}
+// the off-diagonal blocks: the long pairs (by group), the others (by thread)
+template <bool MIXED> static void launch_offdiag_group(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
+    const uint32_t share = group_share(lc), items = pair_slots(lc.cap_pairs) / kPairWindow * (share / kPairGroups);
+    const dim3 grid = grid2(min(items, (uint32_t)lc.sm_count * 28), lc.B);
+    if (lc.use_density) MVDR_LAUNCH((offdiag_group_kernel<MIXED, true>), grid, kPairChunk, 0, st, d, lam, share);
+    else MVDR_LAUNCH((offdiag_group_kernel<MIXED, false>), grid, kPairChunk, 0, st, d, lam, share);
+}
+static void launch_offdiag_group(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
+    if (lc.precision == MVDR_PRECISION_MIXED) launch_offdiag_group<true>(lc, d, lam, st);
+    else launch_offdiag_group<false>(lc, d, lam, st);
+}
+static void launch_offdiag_thread(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
+    const uint32_t share = group_share(lc);
+    const dim3 grid = grid2(min(pair_slots(lc.cap_pairs) / kPairChunk, (uint32_t)lc.sm_count * 16), lc.B);
+    if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH(offdiag_thread_kernel<true>, grid, kPairChunk, 0, st, d, lam, share);
+    else MVDR_LAUNCH(offdiag_thread_kernel<false>, grid, kPairChunk, 0, st, d, lam, share);
+}
+
 cudaError_t launch_assemble(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, bool materialize,
                             cudaStream_t st) {
-    const uint32_t gn = (lc.max_nodes + kDiagNodes - 1) / kDiagNodes;
-    if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH(diag_rhs_kernel<true>, grid2(gn, lc.B), 128, 0, st, d, lam);
-    else MVDR_LAUNCH(diag_rhs_kernel<false>, grid2(gn, lc.B), 128, 0, st, d, lam);
+    launch_diag(lc, d, lam, st);
     if (materialize) {
-        const uint32_t gp = min((lc.cap_pairs + 127) / 128, (uint32_t)lc.sm_count * 8);
-        if (lc.precision == MVDR_PRECISION_MIXED) {
-            MVDR_LAUNCH(offdiag_kernel<true>, grid2(gp, lc.B), 128, 0, st, d, lam);
+        launch_offdiag_group(lc, d, lam, st);
+        launch_offdiag_thread(lc, d, lam, st);
+        if (lc.precision == MVDR_PRECISION_MIXED)
             MVDR_LAUNCH(scale_offdiag_kernel, grid2(scale_grid(lc), lc.B), 128, 0, st, d);
-        } else {
-            MVDR_LAUNCH(offdiag_kernel<false>, grid2(gp, lc.B), 128, 0, st, d, lam);
-        }
     }
     return cudaGetLastError();
 }
 
-// diag_rhs_kernel and offdiag_kernel read the same term records and write
-// disjoint outputs (the diagonal blocks, factors and Jt r; the upper blocks),
-// so they run side by side; the scaling reads both.
+// The diagonal and off-diagonal kernels read the same term records and write
+// disjoint outputs (the diagonal blocks, factors and Jt r; the upper blocks of
+// the long pairs; those of the others), so they run side by side; the scaling
+// reads all of them.
 cudaError_t launch_assemble_forked(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st,
-                                   cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
-    const bool mixed = lc.precision == MVDR_PRECISION_MIXED;
-    cudaError_t e = cudaEventRecord(fork, st);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+                                   const Fork& fork) {
+    cudaError_t e = cudaEventRecord(fork.begin, st);
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(fork.side[k], fork.begin, 0);
     if (e != cudaSuccess) return e;
-    const uint32_t gp = min((lc.cap_pairs + 127) / 128, (uint32_t)lc.sm_count * 8);
-    if (mixed) MVDR_LAUNCH(offdiag_kernel<true>, grid2(gp, lc.B), 128, 0, side, d, lam);
-    else MVDR_LAUNCH(offdiag_kernel<false>, grid2(gp, lc.B), 128, 0, side, d, lam);
-    e = cudaEventRecord(join, side);
-    const uint32_t gn = (lc.max_nodes + kDiagNodes - 1) / kDiagNodes;
-    if (mixed) MVDR_LAUNCH(diag_rhs_kernel<true>, grid2(gn, lc.B), 128, 0, st, d, lam);
-    else MVDR_LAUNCH(diag_rhs_kernel<false>, grid2(gn, lc.B), 128, 0, st, d, lam);
-    // the join is made even after a failed record, so that a capture ends
-    const cudaError_t w = cudaStreamWaitEvent(st, join, 0);
-    if (e == cudaSuccess) e = w;
+    launch_offdiag_thread(lc, d, lam, fork.side[0]);
+    // (a batch fills the GPU: a third branch made 16 x 4096 nodes 1 % slower)
+    launch_offdiag_group(lc, d, lam, lc.B < 4 ? fork.side[1] : st);
+    launch_diag(lc, d, lam, st);
+    // the joins are made even after a failed record, so that a capture ends
+    for (int k = 0; k < 2; ++k) {
+        const cudaError_t r = cudaEventRecord(fork.end[k], fork.side[k]);
+        const cudaError_t w = cudaStreamWaitEvent(st, fork.end[k], 0);
+        if (e == cudaSuccess) e = r != cudaSuccess ? r : w;
+    }
     if (e != cudaSuccess) return e;
-    if (mixed) MVDR_LAUNCH(scale_offdiag_kernel, grid2(scale_grid(lc), lc.B), 128, 0, st, d);
+    if (lc.precision == MVDR_PRECISION_MIXED)
+        MVDR_LAUNCH(scale_offdiag_kernel, grid2(scale_grid(lc), lc.B), 128, 0, st, d);
     return cudaGetLastError();
 }
 
@@ -2440,19 +2802,13 @@ cudaError_t launch_stage(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& l
     const bool scaled = mixed && lc.mode == MVDR_MODE_MATERIALIZED;
     const uint32_t gnode = (lc.max_nodes + kPcgNodeThreads - 1) / kPcgNodeThreads;
     const uint32_t gvec = (6 * lc.max_nodes + 255) / 256;
-    const uint32_t gn = (lc.max_nodes + kDiagNodes - 1) / kDiagNodes;
     switch (stage) {
         case MVDR_STAGE_TERMS: return launch_eval_terms(lc, d, lam, st);
-        case MVDR_STAGE_DIAG:
-            if (mixed) MVDR_LAUNCH(diag_rhs_kernel<true>, grid2(gn, lc.B), 128, 0, st, d, lam);
-            else MVDR_LAUNCH(diag_rhs_kernel<false>, grid2(gn, lc.B), 128, 0, st, d, lam);
+        case MVDR_STAGE_DIAG: launch_diag(lc, d, lam, st); break;
+        case MVDR_STAGE_OFFDIAG:
+            launch_offdiag_group(lc, d, lam, st);
+            launch_offdiag_thread(lc, d, lam, st);
             break;
-        case MVDR_STAGE_OFFDIAG: {
-            const uint32_t gp = min((lc.cap_pairs + 127) / 128, (uint32_t)lc.sm_count * 8);
-            if (mixed) MVDR_LAUNCH(offdiag_kernel<true>, grid2(gp, lc.B), 128, 0, st, d, lam);
-            else MVDR_LAUNCH(offdiag_kernel<false>, grid2(gp, lc.B), 128, 0, st, d, lam);
-            break;
-        }
         case MVDR_STAGE_SPMV:
             return launch_spmv(lc, d, 0, st);
         case MVDR_STAGE_DIRECTION:

@@ -19,12 +19,6 @@ namespace mvdr {
 constexpr int kWarp = 32;
 constexpr uint32_t kInvalid = 0xFFFFFFFFu;
 constexpr uint32_t kTransposedBlock = 0x80000000u;
-// entry-count buckets of the half pairs (bucket 0 = longest; counts of
-// kLenBuckets - 1 or more share bucket 0)
-constexpr uint32_t kLenBuckets = 256;
-__host__ __device__ constexpr uint32_t len_bucket_of(uint32_t len) {
-    return kLenBuckets - 1 - (len < kLenBuckets - 1 ? len : kLenBuckets - 1);
-}
 
 // Element (r, k) of a stored 6x6 JtJ block. The layout keeps row r as three
 // pairs (k = 0-1, 2-3, 4-5) at pair slots r, 6 + r, 12 + r, so six threads that
@@ -38,6 +32,13 @@ __host__ __device__ constexpr uint32_t blk_idx(uint32_t r, uint32_t k) { return 
 // thread reads a block row or a node's direction in one 256-bit load.
 constexpr uint32_t kScaledRow = 8;                  // floats per stored row
 constexpr uint32_t kScaledBlock = 6 * kScaledRow;   // floats per stored block
+
+// order of the off-diagonal kernel's pairs: windows of consecutive pairs, each
+// sorted by entry count, dealt out in chunks of a CTA's pairs
+constexpr uint32_t kPairWindow = 1024, kPairChunk = 128;
+__host__ __device__ constexpr uint32_t pair_slots(uint32_t pairs) {
+    return (pairs + kPairWindow - 1) / kPairWindow * kPairWindow;
+}
 
 constexpr uint32_t kChunkPixels = 2048;  // pixels per compaction CTA (256 threads x 8)
 
@@ -278,15 +279,14 @@ struct InstDesc {
     uint32_t* row_count;    // [N+1] entries (j, t) with j > i per row
     uint32_t* row_offset;   // [N+1]
     uint32_t* np_index;     // [K2 cap]
-    float2* np_w;           // [K2 cap] skinning weights of the pair's (i, j) nodes in the entry's term
+    double* np_scale;       // [K2 cap] w_i w_j of the entry's term (0 for smooth), the exact product
     uint32_t* upper_count;  // [N+1]
     uint32_t* half_offset;  // [N+1]
     uint32_t* tmp_key;      // [K2 cap] per-row unique pairs before compaction
     uint32_t* tmp_start;    // [K2 cap]
     uint32_t* half_key;     // [P cap]
     uint2* half_range;      // [P cap]
-    uint32_t* pair_order;   // [P cap] half pairs grouped by entry count, longest first
-    uint32_t* len_bucket;   // [2 * kLenBuckets] pairs per entry-count bucket, then scatter cursors
+    uint32_t* pair_order;   // [pair_slots(P cap)] half pairs, about longest first (kInvalid: no pair)
     uint32_t* lower_count;  // [N+1]
     uint32_t* lower_cursor; // [N]
     uint32_t* blkrow_offset;// [N+1]
@@ -411,12 +411,18 @@ cudaError_t launch_build_index(const LaunchCfg& lc, InstDesc* d_inst, cudaStream
 cudaError_t launch_eval_terms(const LaunchCfg& lc, InstDesc* d_inst, const mvdr_penalty& lam, cudaStream_t st);
 cudaError_t launch_assemble(const LaunchCfg& lc, InstDesc* d_inst, const mvdr_penalty& lam, bool materialize,
                             cudaStream_t st);
-// The materialised assembly with the off-diagonal blocks on `side` while the
-// diagonal blocks run on `st` (forked after the work queued on `st`, joined
-// back before the scaling, which needs both); inside a stream capture the
-// two become parallel branches of the graph.
+// The streams beside the solve's stream, and the events that fork them from it
+// and join them back; a batch owns one.
+struct Fork {
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t begin = nullptr, end[2] = {nullptr, nullptr};
+};
+// The materialised assembly with the off-diagonal blocks on the side streams
+// while the diagonal blocks run on `st` (forked after the work queued on `st`,
+// joined back before the scaling, which needs all); inside a stream capture they
+// become parallel branches of the graph.
 cudaError_t launch_assemble_forked(const LaunchCfg& lc, InstDesc* d_inst, const mvdr_penalty& lam, cudaStream_t st,
-                                   cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
+                                   const Fork& fork);
 cudaError_t launch_energy(const LaunchCfg& lc, InstDesc* d_inst, uint32_t slot, cudaStream_t st);
 cudaError_t launch_pcg(const LaunchCfg& lc, InstDesc* d_inst, const mvdr_penalty& lam, uint32_t iters, uint32_t gn,
                        cudaStream_t st);

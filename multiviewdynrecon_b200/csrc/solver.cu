@@ -71,9 +71,11 @@ Batch::~Batch() {
         if (o.mem) cudaFree(o.mem);
     if (d_inst) cudaFree(d_inst);
     if (d_bars) cudaFree(d_bars);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
+    if (fork.begin) cudaEventDestroy(fork.begin);
+    for (int k = 0; k < 2; ++k) {
+        if (fork.end[k]) cudaEventDestroy(fork.end[k]);
+        if (fork.side[k]) cudaStreamDestroy(fork.side[k]);
+    }
     if (arena) cudaFree(arena);
     for (auto* v : views) delete v;
 }
@@ -126,15 +128,14 @@ static size_t layout_instance(Arena& a, InstDesc& I, const LaunchCfg& lc, uint32
     I.row_count = a.take<uint32_t>(N + 1);
     I.row_offset = a.take<uint32_t>(N + 1);
     I.np_index = a.take<uint32_t>(lc.cap_k2);
-    I.np_w = a.take<float2>(lc.cap_k2);
+    I.np_scale = a.take<double>(lc.cap_k2);
     I.upper_count = a.take<uint32_t>(N + 1);
     I.half_offset = a.take<uint32_t>(N + 1);
     I.tmp_key = a.take<uint32_t>(lc.cap_k2);
     I.tmp_start = a.take<uint32_t>(lc.cap_k2);
     I.half_key = a.take<uint32_t>(lc.cap_pairs);
     I.half_range = a.take<uint2>(lc.cap_pairs);
-    I.pair_order = a.take<uint32_t>(lc.cap_pairs);
-    I.len_bucket = a.take<uint32_t>(2 * kLenBuckets);
+    I.pair_order = a.take<uint32_t>(pair_slots(lc.cap_pairs));
     I.lower_count = a.take<uint32_t>(N + 1);
     I.lower_cursor = a.take<uint32_t>(N + 1);
     I.blkrow_offset = a.take<uint32_t>(N + 1);
@@ -293,9 +294,11 @@ static int create_batch(const mvdr_config* cfg, uint32_t B, Batch** out) {
     e = cudaMemset(b->arena, 0, b->arena_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_inst, sizeof(InstDesc) * B);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_bars, sizeof(uint32_t) * 32 * B);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork.begin, cudaEventDisableTiming);
+    for (int k = 0; k < 2; ++k) {
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->fork.side[k], cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork.end[k], cudaEventDisableTiming);
+    }
     if (e != cudaSuccess) {
         delete b;
         return fail(MVDR_ECUDA, std::string("workspace setup failed: ") + cudaGetErrorString(e));
@@ -663,7 +666,7 @@ static int enqueue_iteration(Batch& b, uint32_t iter, uint32_t pcg, cudaStream_t
     {
         NvtxRange r("mvdr/assemble");
         if (b.cfg.mode == MVDR_MODE_MATERIALIZED)
-            CU(launch_assemble_forked(b.lc, b.d_inst, lam, st, b.side, b.ev_fork, b.ev_join));
+            CU(launch_assemble_forked(b.lc, b.d_inst, lam, st, b.fork));
         else
             CU(launch_assemble(b.lc, b.d_inst, lam, false, st));
     }
