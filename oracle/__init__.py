@@ -34,9 +34,9 @@ _ref_lib = None
 
 def build():
     subprocess.run(["make", "-s", "-C", _HERE], check=True)
-    # the reference-pinning harness needs the reference tree; elsewhere the
-    # library built here (oracle/_ref) is used as it is
-    if os.path.isdir(REFERENCE_TREE):
+    # the reference-pinning harness needs the reference's headers; elsewhere
+    # the library built here (oracle/_ref) is used as it is
+    if any("EncodeUtils.h" in files for _, _, files in os.walk(REFERENCE_TREE)):
         subprocess.run(["make", "-s", "-C", _HERE, "ref", f"REF={REFERENCE_TREE}"], check=True)
 
 
