@@ -1319,6 +1319,9 @@ __global__ void __launch_bounds__(128) pcg_unscale_kernel(const InstDesc* insts)
 // holds d.q of the current iteration; the scaled SpMV also stores r.q and q.q
 // (kRegRq, kRegQq), from which the fused update forms the next delta.
 constexpr uint32_t kRegDelta = 1, kRegDq = 3, kRegRq = 5, kRegQq = 6;
+// the resident PCG's d.q, r.q and q.q by parity (a CTA may still read one
+// iteration's while another stores the next one's)
+constexpr uint32_t kRegResident = 7;
 
 template <class T>
 __device__ inline void store_block_partial(const InstDesc& I, uint32_t region, T v, uint32_t slot = 0xFFFFFFFFu) {
@@ -1355,6 +1358,25 @@ __device__ inline void store_block_partials3(const InstDesc& I, uint32_t r0, T v
     }
 }
 
+// A region's partials summed by one warp: lane l takes l, l + 32, ... in turn,
+// then a butterfly. The loads of kPartialBatch steps are issued together: one
+// after the other, the 64 steps of a 32,768-node instance cost 10 us in every
+// update.
+constexpr uint32_t kPartialBatch = 8;
+
+template <class T> __device__ inline T sum_partials(const double* p, uint32_t n) {
+    T s = 0;
+    for (uint32_t base = lane_id(); base < n; base += 32 * kPartialBatch) {
+        double v[kPartialBatch];
+#pragma unroll
+        for (uint32_t q = 0; q < kPartialBatch; ++q) v[q] = base + 32 * q < n ? __ldcg(p + base + 32 * q) : 0.0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPartialBatch; ++q)
+            if (base + 32 * q < n) s += (T)v[q];
+    }
+    return warp_sum(s);
+}
+
 // The sums of the partials of four regions (warp w sums regions w, w + warps,
 // ...; each in a fixed order), in every thread. blockDim.x >= 64.
 template <class T>
@@ -1363,10 +1385,7 @@ __device__ inline void sum_four_block_partials(const InstDesc& I, const uint32_t
     __shared__ T total[4];
     const uint32_t warps = blockDim.x >> 5;
     for (uint32_t q = threadIdx.x >> 5; q < 4; q += warps) {
-        const double* p = I.partials + (size_t)reg[q] * I.part_stride;
-        T s = 0;
-        for (uint32_t c = lane_id(); c < cnt[q]; c += 32) s += (T)__ldcg(p + c);
-        s = warp_sum(s);
+        const T s = sum_partials<T>(I.partials + (size_t)reg[q] * I.part_stride, cnt[q]);
         if (lane_id() == 0) total[q] = s;
     }
     __syncthreads();
@@ -1788,6 +1807,10 @@ __global__ void __launch_bounds__(6 * kTileSplit * kTileRows) pcg_spmv_scaled_ke
     store_block_partials3<double>(I, kRegDq, part, kRegRq, prq, kRegQq, pqq);
 }
 
+// PCG init and update: a thread per node, 64 nodes per CTA, so that the small
+// grid spreads over every SM
+constexpr uint32_t kPcgNodeThreads = 64;
+
 // blockPCGSecondUpdateKernel (BlockPCG.cuh:120-161): alpha = delta / d.q,
 // x += alpha d, r -= alpha q, s = M^-1 r, delta_new = r.s (beta follows in
 // the next direction). A thread per node; the grid covers every node. The
@@ -1816,8 +1839,9 @@ __global__ void __launch_bounds__(256) pcg_update_kernel(const InstDesc* insts, 
     using T = typename PV::T;
     using T2 = typename Pair<T>::type;
     constexpr int kPre = SCALED ? 1 : (MIXED ? 21 : 36);  // Cholesky factor / inverse entries
-    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool has = node < I.N;
+    // (the launch may add two warps that only sum partials)
+    const uint32_t node = blockIdx.x * kPcgNodeThreads + threadIdx.x;
+    const bool has = threadIdx.x < kPcgNodeThreads && node < I.N;
     T xv[6], dv[6], rv[6], qv[6];
     T pre[kPre];
     if (has) {
@@ -2162,6 +2186,365 @@ __global__ void __launch_bounds__(kPersistThreads, 3) pcg_persistent_kernel(cons
             chol_backward(L, xh, x);
 #pragma unroll
             for (int q = 0; q < 6; ++q) I.x_d[6 * (size_t)node + q] = x[q];
+        }
+    }
+}
+
+// ------------------------------------------------------- resident PCG ---
+// The whole PCG solve of one instance of up to kResidentRows nodes per SM in one
+// cooperative launch (mixed precision, materialised, one instance, the default
+// tile shape, no tolerance). A 4096-node solve's operator is 8 MB: every CTA keeps
+// the blocks of its 32 block rows in shared memory for all iterations, and with
+// each entry the state (r^, d) of the entry's column, which it updates itself: an
+// iteration needs one grid barrier instead of two, after which every CTA reads the
+// partial sums and the q of its columns. The tiles, the products, the reductions
+// and their order are those of pcg_spmv_scaled_kernel<16, 2, 0> and
+// pcg_update_kernel with their roundings written out, so the increments are the
+// same to the bit.
+// An iteration takes 6.9 us against 13.5 for the two launches with their gaps
+// (4096-node frame; the whole solve 2300 -> 1634 us, a 500-node frame 1445 -> 1225).
+constexpr uint32_t kResidentRows = 32, kResidentTile = 16;   // block rows per CTA and per tile of the SpMV
+constexpr uint32_t kResidentThreads = 12 * kResidentRows;    // 12 threads per block row, as the tile shape
+constexpr uint32_t kResidentEntries = 736;                   // entries kept in shared memory (the others in global memory)
+// every CTA is resident, so a wait ends within microseconds; the limit only
+// keeps a fault elsewhere from hanging the GPU
+constexpr uint64_t kResidentWaitNs = 2000ull * 1000 * 1000;
+constexpr uint32_t kResidentGather = 8;                      // column values per thread loaded before the sums are known
+
+struct ResidentSmem {
+    double r[kResidentRows + kResidentEntries][6];   // own rows, then one slot per entry
+    double d[kResidentRows + kResidentEntries][6];
+    float df[kResidentRows + kResidentEntries][6];
+    float blk[kResidentEntries][36];                 // the entry's stored block, six rows of six
+    uint32_t col[kResidentRows + kResidentEntries];  // global column of a slot
+    uint32_t upper0[kResidentRows];                  // first entry of each own row that lies above the diagonal
+    float x[kResidentThreads][7];                    // the tiles' exchange
+    double ws[3][kResidentThreads / 32];
+    double total[4];
+    uint32_t row0[kResidentRows + 1];                // first entry of each own row
+    int ok;
+};
+static_assert(sizeof(ResidentSmem) <= 227 * 1024, "shared memory of one SM");
+
+// a . x with the roundings of the launched form's a[0] * x[0] + ... + a[5] * x[5],
+// written out so that they do not depend on the code around it
+__device__ inline float six_products(const float (&a)[6], const float (&x)[6]) {
+    float s = __fmaf_rn(a[0], x[0], __fmul_rn(a[1], x[1]));
+#pragma unroll
+    for (int k = 2; k < 6; ++k) s = __fmaf_rn(a[k], x[k], s);
+    return s;
+}
+
+// All CTAs of the grid arrive; false (and the instance flagged) when the wait
+// exceeds limit_ns.
+__device__ inline bool resident_barrier(const InstDesc& I, ResidentSmem& m, uint32_t target, uint64_t limit_ns) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(I.pcg_bar, 1u);
+        int ok = 1;
+        uint64_t t0 = 0;
+        for (uint32_t spins = 0; ld_acquire_u32(I.pcg_bar) < target; ++spins) {
+            if ((spins & 255u) != 255u) continue;
+            const uint64_t now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > limit_ns) {
+                ok = 0;
+                set_error(I, kErrWaitTimeout);
+                break;
+            }
+        }
+        __threadfence();
+        m.ok = ok;
+    }
+    __syncthreads();
+    return m.ok != 0;
+}
+
+__global__ void __launch_bounds__(kResidentThreads, 1) pcg_resident_kernel(const InstDesc* insts, uint32_t iters,
+                                                                           uint32_t nd, uint32_t nq, uint32_t gn,
+                                                                           uint64_t limit_ns) {
+    extern __shared__ __align__(16) unsigned char s_resident[];
+    ResidentSmem& m = *reinterpret_cast<ResidentSmem*>(s_resident);
+    const InstDesc& I = insts[0];
+    const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5, G = gridDim.x;
+    const uint32_t base = blockIdx.x * kResidentRows;
+    const uint32_t rows = base < I.N ? min(kResidentRows, I.N - base) : 0u;
+    const bool index_ok = index_complete(I);
+    // ---- the CTA's rows: entries without the (identity) diagonal
+    if (t <= kResidentRows) {
+        const uint32_t row = min(base + t, I.N);
+        m.row0[t] = base < I.N ? I.blkrow_offset[row] - I.blkrow_offset[base] : 0u;
+    }
+    if (t < kResidentRows) {
+        m.col[t] = base + t;
+        m.upper0[t] = t < rows ? I.blkrow_offset[base + t] - I.blkrow_offset[base] + I.lower_count[base + t] : 0u;
+    }
+    __syncthreads();
+    const uint32_t entries = index_ok ? m.row0[kResidentRows] : 0u;
+    const uint32_t first_entry = base < I.N ? I.blkrow_offset[base] + base : 0u;  // (its diagonal entry)
+    const uint32_t lr = t / 12, half = (t / 6) % 2, rr = t % 6;
+    const bool computes = lr < rows && index_ok;
+    // entries past the shared ones keep their column state in this scratch
+    double* far_r = I.resident + 12 * (size_t)(base < I.N ? I.blkrow_offset[base] : 0u);
+    if (computes) {
+        const uint32_t e1 = m.row0[lr + 1];
+        for (uint32_t e = m.row0[lr] + half; e < e1; e += 2) {
+            const uint2 ent = I.bsr_ent[first_entry + lr + 1 + e];  // (each row's diagonal entry precedes its others)
+            if (e >= kResidentEntries) continue;
+            float av[8];
+            load8f(I.bsr_s + kScaledBlock * (size_t)(ent.x & ~kTransposedBlock) + kScaledRow * rr, av);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) m.blk[e][6 * rr + k] = av[k];
+            if (rr == 0) m.col[kResidentRows + e] = ent.y;
+        }
+    }
+    // ---- init: r^ = L^-1 b, x^ = 0, delta_0 (pcg_init_kernel); lane = own node
+    const uint32_t node = base + t;
+    const bool owner = t < rows;
+    double x[6] = {0, 0, 0, 0, 0, 0};
+    if (warp == 0) {
+        double part = 0;
+        if (owner) {
+            double bv[6], rv[6], L[21];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) bv[i] = I.jtr_d[6 * (size_t)node + i];
+#pragma unroll
+            for (int q = 0; q < 21; ++q) L[q] = I.chol[21 * (size_t)node + q];
+            chol_forward(L, bv, rv);
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                m.r[t][i] = rv[i];
+                m.d[t][i] = rv[i];
+                m.df[t][i] = (float)rv[i];
+                I.r_d[6 * (size_t)node + i] = rv[i];
+                part = __fma_rn(rv[i], rv[i], part);
+            }
+        }
+        part = warp_sum(part);
+        if (lane == 0) I.partials[(size_t)kRegDelta * I.part_stride + blockIdx.x] = part;
+    }
+    if (blockIdx.x == 0) {
+        if (t == 0) I.counts->pcg_stop = 0u;
+        if (gn < kPcgHistRows)
+            for (uint32_t k = t; k < MVDR_PCG_HISTORY; k += kResidentThreads)
+                I.pcg_hist[(size_t)gn * MVDR_PCG_HISTORY + k] = __longlong_as_double(0x7ff8000000000000ll);
+    }
+    uint32_t passed = 0;
+    if (!resident_barrier(I, m, ++passed * G, limit_ns)) return;
+    // the columns' r^ and d of the first iteration (beta = 0: d = r^)
+    for (uint32_t i = t; i < 6 * entries; i += kResidentThreads) {
+        const uint32_t e = i / 6, c = i % 6;
+        if (e < kResidentEntries) {
+            const double v = __ldcg(I.r_d + 6 * (size_t)m.col[kResidentRows + e] + c);
+            m.r[kResidentRows + e][c] = v;
+            m.d[kResidentRows + e][c] = v;
+            m.df[kResidentRows + e][c] = (float)v;
+        }
+    }
+    // (the far entries: thread by thread as they are read below)
+    if (computes && entries > kResidentEntries) {
+        const uint32_t e1 = m.row0[lr + 1];
+        for (uint32_t e = m.row0[lr] + half; e < e1; e += 2) {
+            if (e < kResidentEntries) continue;
+            const uint32_t col = I.bsr_ent[first_entry + lr + 1 + e].y;
+            const double v = __ldcg(I.r_d + 6 * (size_t)col + rr);
+            far_r[12 * (size_t)e + rr] = v;
+            far_r[12 * (size_t)e + 6 + rr] = v;
+        }
+    }
+    __syncthreads();
+    for (uint32_t it = 0; it < iters; ++it) {
+        const uint32_t parity = it & 1u;
+        double* q_out = parity ? I.s_d : I.q_d;
+        // ---- q^ = A^ d^ of the own rows (pcg_spmv_scaled_kernel<16, 2, 0>)
+        float acc = 0.f;
+        float col_acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (computes) {
+            // a row's lower entries come first: row rr of the stored A_ji times
+            // d_j(rr) adds to all six rows; an upper entry gives row rr directly
+            const uint32_t e1 = m.row0[lr + 1], u1 = min(m.upper0[lr], e1);
+            uint32_t e = m.row0[lr] + half;
+#pragma unroll 2
+            for (; e < min(u1, kResidentEntries); e += 2) {
+                const float2* b2 = reinterpret_cast<const float2*>(&m.blk[e][6 * rr]);
+                const float2 b01 = b2[0], b23 = b2[1], b45 = b2[2];
+                const float av[6] = {b01.x, b01.y, b23.x, b23.y, b45.x, b45.y};
+                const float xr = m.df[kResidentRows + e][rr];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) col_acc[k] += av[k] * xr;
+            }
+#pragma unroll 2
+            for (; e < min(e1, kResidentEntries); e += 2) {
+                if (e < u1) break;  // (the lower entries reach past the shared ones)
+                const float2* b2 = reinterpret_cast<const float2*>(&m.blk[e][6 * rr]);
+                const float2* x2 = reinterpret_cast<const float2*>(m.df[kResidentRows + e]);
+                const float2 b01 = b2[0], b23 = b2[1], b45 = b2[2], x01 = x2[0], x23 = x2[1], x45 = x2[2];
+                const float av[6] = {b01.x, b01.y, b23.x, b23.y, b45.x, b45.y};
+                const float xv[6] = {x01.x, x01.y, x23.x, x23.y, x45.x, x45.y};
+                acc += six_products(av, xv);
+            }
+            for (; e < e1; e += 2) {  // entries past the shared ones
+                const uint32_t pos = I.bsr_ent[first_entry + lr + 1 + e].x;
+                float av[8], xv[6];
+                load8f(I.bsr_s + kScaledBlock * (size_t)(pos & ~kTransposedBlock) + kScaledRow * rr, av);
+                const double* dc = far_r + 12 * (size_t)e + 6;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) xv[k] = (float)dc[k];
+                if (e < u1) {
+                    const float xr = (float)dc[rr];
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) col_acc[k] += av[k] * xr;
+                } else {
+                    const float a6[6] = {av[0], av[1], av[2], av[3], av[4], av[5]};
+                    acc += six_products(a6, xv);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) m.x[t][k] = col_acc[k];
+            m.x[t][6] = acc;
+        }
+        __syncthreads();
+        double part = 0, prq = 0, pqq = 0;  // d.q, r.q, q.q
+        if (computes && half == 0) {
+            acc = 0.f;
+#pragma unroll
+            for (uint32_t hh = 0; hh < 2; ++hh) {
+                const float(*mine)[7] = m.x + lr * 12 + hh * 6;
+                acc += mine[rr][6];
+#pragma unroll
+                for (int c = 0; c < 6; ++c) acc += mine[c][rr];
+            }
+            const double dv = m.d[lr][rr];
+            const double q = dv + (double)acc;
+            q_out[6 * (size_t)(base + lr) + rr] = q;
+            part = __dmul_rn(dv, q);
+            prq = __dmul_rn(m.r[lr][rr], q);
+            pqq = __dmul_rn(q, q);
+        }
+        part = warp_sum(part);
+        prq = warp_sum(prq);
+        pqq = warp_sum(pqq);
+        if (lane == 0) {
+            m.ws[0][warp] = part;
+            m.ws[1][warp] = prq;
+            m.ws[2][warp] = pqq;
+        }
+        __syncthreads();
+        constexpr uint32_t kTiles = kResidentRows / kResidentTile, kTileWarps = kResidentThreads / 32 / kTiles;
+        if (t < 3 * kTiles) {  // a tile's partials, as its CTA of the launched form stores them
+            const uint32_t region = t % 3, tile = t / 3;
+            double sum = 0;
+            for (uint32_t w = 0; w < kTileWarps; ++w) sum += m.ws[region][tile * kTileWarps + w];
+            I.partials[(size_t)(kRegResident + 3 * parity + region) * I.part_stride + blockIdx.x * kTiles + tile] = sum;
+        }
+        if (!resident_barrier(I, m, ++passed * G, limit_ns)) return;
+        // ---- the partials' sums (warps 0-3, their loads first) beside the
+        // columns' q
+        constexpr uint32_t kSteps = 8;
+        double pv[kSteps];
+        const uint32_t count = warp == 0 ? nd : nq;
+        const double* p = I.partials + (size_t)(warp == 0 ? kRegDelta + parity : kRegResident + 3 * parity + warp - 1) * I.part_stride;
+        auto load_partial = [&](uint32_t c) {
+            if (c >= count) return 0.0;
+            if (warp != 0) return __ldcg(p + c);
+            // (delta partials are per 32 nodes here and per 64 in the launched form)
+            return __ldcg(p + 2 * c) + (2 * c + 1 < G ? __ldcg(p + 2 * c + 1) : 0.0);
+        };
+        if (warp < 4) {
+#pragma unroll
+            for (uint32_t g = 0; g < kSteps; ++g) pv[g] = load_partial(lane + 32 * g);
+        }
+        double qv[kResidentGather];
+        const uint32_t near = 6 * min(entries, kResidentEntries);
+#pragma unroll
+        for (uint32_t g = 0; g < kResidentGather; ++g) {
+            const uint32_t i = t + g * kResidentThreads;
+            qv[g] = i < near ? __ldcg(q_out + 6 * (size_t)m.col[kResidentRows + i / 6] + i % 6) : 0.0;
+        }
+        if (warp < 4) {
+            double sum = 0;
+#pragma unroll
+            for (uint32_t g = 0; g < kSteps; ++g)
+                if (lane + 32 * g < count) sum += pv[g];
+            for (uint32_t c = lane + 32 * kSteps; c < count; c += 32) sum += load_partial(c);
+            sum = warp_sum(sum);
+            if (lane == 0) m.total[warp] = sum;
+        }
+        __syncthreads();
+        const double delta = m.total[0], dq = m.total[1], rq = m.total[2], qq = m.total[3];
+        if (blockIdx.x == 0 && t == 0) {
+            if (it == 0) I.counts->pcg_delta0 = delta;
+            if (gn < kPcgHistRows && it < MVDR_PCG_HISTORY) I.pcg_hist[(size_t)gn * MVDR_PCG_HISTORY + it] = delta;
+        }
+        // ---- alpha, x^, r^, the next direction (pcg_update_kernel)
+        const double alpha = pcg_alpha<double>(I, delta, dq, blockIdx.x == 0);
+        const double dnext = __fma_rn(__dmul_rn(alpha, alpha), qq, __fma_rn(-2.0 * alpha, rq, delta));
+        const double beta = delta != (double)0 ? dnext / delta : (double)0;
+        if (warp == 0) {
+            double dsum = 0;
+            if (owner) {
+                double rv[6];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                    const double dv = m.d[t][i];
+                    const double q = __ldcg(q_out + 6 * (size_t)node + i);
+                    x[i] = __fma_rn(alpha, dv, x[i]);
+                    rv[i] = __fma_rn(-alpha, q, m.r[t][i]);
+                    const double dn = __fma_rn(beta, dv, rv[i]);
+                    m.r[t][i] = rv[i];
+                    m.d[t][i] = dn;
+                    m.df[t][i] = (float)dn;
+                }
+                // (the launched form's order of roundings for a sum that starts at zero)
+                dsum = __fma_rn(rv[0], rv[0], __dmul_rn(rv[1], rv[1]));
+#pragma unroll
+                for (int i = 2; i < 6; ++i) dsum = __fma_rn(rv[i], rv[i], dsum);
+            }
+            dsum = warp_sum(dsum);
+            if (lane == 0) I.partials[(size_t)(kRegDelta + (parity ^ 1u)) * I.part_stride + blockIdx.x] = dsum;
+        }
+        auto advance = [&](double& r, double& d, double q) {
+            r = __fma_rn(-alpha, q, r);
+            d = __fma_rn(beta, d, r);
+        };
+#pragma unroll
+        for (uint32_t g = 0; g < kResidentGather; ++g) {
+            const uint32_t i = t + g * kResidentThreads;
+            if (i < near) {
+                const uint32_t slot = kResidentRows + i / 6, c = i % 6;
+                advance(m.r[slot][c], m.d[slot][c], qv[g]);
+                m.df[slot][c] = (float)m.d[slot][c];
+            }
+        }
+        for (uint32_t i = t + kResidentGather * kResidentThreads; i < near; i += kResidentThreads) {
+            const uint32_t slot = kResidentRows + i / 6, c = i % 6;
+            advance(m.r[slot][c], m.d[slot][c], __ldcg(q_out + 6 * (size_t)m.col[slot] + c));
+            m.df[slot][c] = (float)m.d[slot][c];
+        }
+        if (computes && entries > kResidentEntries) {
+            const uint32_t e1 = m.row0[lr + 1];
+            for (uint32_t e = m.row0[lr] + half; e < e1; e += 2) {
+                if (e < kResidentEntries) continue;
+                const uint32_t col = I.bsr_ent[first_entry + lr + 1 + e].y;
+                advance(far_r[12 * (size_t)e + rr], far_r[12 * (size_t)e + 6 + rr], __ldcg(q_out + 6 * (size_t)col + rr));
+            }
+        }
+        __syncthreads();
+    }
+    // ---- x = L^-T x^ (pcg_unscale_kernel); r^ and the direction as the launched form leaves them
+    if (owner) {
+        double L[21], xo[6];
+#pragma unroll
+        for (int q = 0; q < 21; ++q) L[q] = I.chol[21 * (size_t)node + q];
+        chol_backward(L, x, xo);
+        double* d_out = PcgVec<true>::d(I, (int)(iters & 1u));
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            I.x_d[6 * (size_t)node + i] = xo[i];
+            I.r_d[6 * (size_t)node + i] = m.r[t][i];
+            d_out[6 * (size_t)node + i] = m.d[t][i];
+            I.df[kScaledRow * (size_t)node + i] = m.df[t][i];
         }
     }
 }
@@ -2647,9 +3030,11 @@ cudaError_t launch_energy(const LaunchCfg& lc, InstDesc* d, uint32_t slot, cudaS
     return cudaGetLastError();
 }
 
-// PCG init and update: a thread per node in CTAs of 64, so that the small
-// grid spreads over every SM
-constexpr uint32_t kPcgNodeThreads = 64;
+// Threads of the fused update: a warp per partial region, or (in batches, whose
+// other instances fill the SMs meanwhile) two warps with two regions each. us:
+// 32,768-node frame 8.3 / 11.7, 4096-node frame 3.4 / 4.0; uneven batch's solve, ms,
+// 8.15 / 8.06.
+static uint32_t fused_update_threads(const LaunchCfg& lc) { return kPcgNodeThreads * (lc.B < 4 ? 2 : 1); }
 
 // CTAs per instance of the SpMV launch with the current shape
 static uint32_t spmv_grid(const LaunchCfg& lc) {
@@ -2690,11 +3075,53 @@ static cudaError_t launch_pcg_persistent(const LaunchCfg& lc, InstDesc* d, uint3
     return e;
 }
 
+// the resident form's conditions; the rest runs launch by launch
+static bool resident_pcg(const LaunchCfg& lc) {
+    return lc.resident && lc.B == 1 && lc.spmv_shape == 0 && lc.pcg_tol == 0.f;
+}
+
+bool resident_pcg_fits(const LaunchCfg& lc) {
+    if (lc.B != 1 || lc.precision != MVDR_PRECISION_MIXED || lc.mode != MVDR_MODE_MATERIALIZED) return false;
+    if (lc.max_nodes > kResidentRows * (uint32_t)lc.sm_count) return false;
+    int nb = 0;
+    cudaError_t e = cudaFuncSetAttribute(pcg_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(ResidentSmem));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pcg_resident_kernel, kResidentThreads, sizeof(ResidentSmem));
+    if (e != cudaSuccess) cudaGetLastError();  // (not an error of the caller's)
+    return e == cudaSuccess && nb > 0;
+}
+
+static cudaError_t launch_pcg_resident(const LaunchCfg& lc, InstDesc* d, uint32_t iters, uint32_t gn, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(lc.pcg_bars, 0, sizeof(uint32_t) * 32 * lc.B, st);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((lc.max_nodes + kResidentRows - 1) / kResidentRows);
+    cfg.blockDim = dim3(kResidentThreads);
+    cfg.dynamicSmemBytes = sizeof(ResidentSmem);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const uint32_t nd = (lc.max_nodes + kPcgNodeThreads - 1) / kPcgNodeThreads;
+    e = cudaLaunchKernelEx(&cfg, pcg_resident_kernel, (const InstDesc*)d, iters, nd, spmv_grid(lc), gn, kResidentWaitNs);
+    if (e == cudaSuccess) count_launch();
+    return e;
+}
+
 cudaError_t launch_pcg(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, uint32_t iters, uint32_t gn,
                        cudaStream_t st) {
     // the convergence check runs in the launched form only
     if (lc.pcg_persistent && lc.mode == MVDR_MODE_MATERIALIZED && lc.pcg_tol == 0.f)
         return launch_pcg_persistent(lc, d, iters, st);
+    if (resident_pcg(lc) && iters > 0) {
+        const cudaError_t e = launch_pcg_resident(lc, d, iters, gn, st);
+        // (a context with fewer SMs than the device runs launch by launch)
+        if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+        cudaGetLastError();
+    }
     const bool mixed = lc.precision == MVDR_PRECISION_MIXED;
     // the update's and direction's grids cover every node / element
     const uint32_t gnode = (lc.max_nodes + kPcgNodeThreads - 1) / kPcgNodeThreads;
@@ -2729,7 +3156,7 @@ cudaError_t launch_pcg(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam
             if (e != cudaSuccess) return e;
             nq = spmv_grid(lc);
         }
-        if (scaled) MVDR_LAUNCH((pcg_update_kernel<true, true, true>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, parity, gnode, nq, gn, it);
+        if (scaled) MVDR_LAUNCH((pcg_update_kernel<true, true, true>), grid2(gnode, lc.B), fused_update_threads(lc), 0, st, d, parity, gnode, nq, gn, it);
         else if (mixed) MVDR_LAUNCH((pcg_update_kernel<true, false, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, parity, gnode, nq, gn, it);
         else MVDR_LAUNCH((pcg_update_kernel<false, false, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, parity, gnode, nq, gn, it);
     }
@@ -2819,7 +3246,7 @@ cudaError_t launch_stage(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& l
             break;
         case MVDR_STAGE_PCG_UPDATE:
             // (the form the solve runs; no residual history)
-            if (scaled) MVDR_LAUNCH((pcg_update_kernel<true, true, true>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, 0, gnode, spmv_grid(lc), ~0u, 1u);
+            if (scaled) MVDR_LAUNCH((pcg_update_kernel<true, true, true>), grid2(gnode, lc.B), fused_update_threads(lc), 0, st, d, 0, gnode, spmv_grid(lc), ~0u, 1u);
             else if (mixed) MVDR_LAUNCH((pcg_update_kernel<true, false, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, 0, gnode, spmv_grid(lc), ~0u, 1u);
             else MVDR_LAUNCH((pcg_update_kernel<false, false, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, 0, gnode, spmv_grid(lc), ~0u, 1u);
             break;

@@ -343,7 +343,8 @@ struct InstDesc {
     double* d0_d;
     double* d1_d;
     float* jp;              // matrix-free scratch: J.p per scalar term
-    double* partials;       // per-CTA partial sums: 4 regions of part_stride
+    double* partials;       // per-CTA partial sums: 13 regions of part_stride
+    double* resident;       // resident PCG: column state of the entries past the shared ones [12 per entry]
     uint32_t part_stride;   // >= the CTAs per instance of any launch
     uint32_t* pcg_bar;      // persistent PCG: this instance's barrier counter (batch-owned)
     double* energy;         // [max GN iterations + 1]
@@ -378,6 +379,7 @@ struct LaunchCfg {
     uint32_t wait_extra_arrivals;
     float pcg_tol;  // PCG convergence tolerance (0: fixed iteration count)
     int recompute_jr;  // matrix-free products re-derive the pixel terms' records
+    int resident;      // the PCG may run as one resident launch (resident_pcg_fits)
 };
 
 constexpr uint32_t kPcgHistRows = 64;  // GN iterations whose PCG residuals are kept
@@ -392,6 +394,10 @@ void count_launch();
 
 // co-resident CTAs of the persistent PCG kernel on this device (0 on error)
 uint32_t persistent_pcg_grid(int mixed, int sm_count);
+
+// whether this configuration's PCG can run as one launch with the operator kept
+// in shared memory
+bool resident_pcg_fits(const LaunchCfg& lc);
 
 // raise the dynamic shared-memory limit of the segment-sort kernels
 cudaError_t set_index_smem_limits(size_t seg_bytes);

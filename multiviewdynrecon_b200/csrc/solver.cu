@@ -181,8 +181,9 @@ static size_t layout_instance(Arena& a, InstDesc& I, const LaunchCfg& lc, uint32
     // J.p per scalar term of the matrix-free operator (double in mixed precision)
     I.jp = lc.mode == MVDR_MODE_MATRIX_FREE ? a.take<float>(6 * (size_t)lc.cap_terms) : nullptr;
     // region 0: energy; 1, 2: PCG delta by iteration parity; 3: d.q; 4: the
-    // density term's energy
-    I.partials = a.take<double>(7 * (size_t)partial_slots);
+    // density term's energy; 5, 6: r.q, q.q; 7-12: the resident PCG's
+    I.partials = a.take<double>(13 * (size_t)partial_slots);
+    I.resident = lc.resident ? a.take<double>(12 * 2 * (size_t)lc.cap_pairs) : nullptr;
     I.part_stride = partial_slots;
     I.energy = a.take<double>(64);
     I.node_err_acc = a.take<unsigned long long>(2 * N);
@@ -267,6 +268,7 @@ static int create_batch(const mvdr_config* cfg, uint32_t B, Batch** out) {
     lc.pcg_tol = cfg->pcg_tolerance;
     lc.recompute_jr = cfg->recompute_jacobians ? 1 : 0;
     lc.sm_count = prop.multiProcessorCount;
+    lc.resident = resident_pcg_fits(lc) ? 1 : 0;
 
     const size_t smem_seg = (size_t)lc.cap_seg * 4;
     if (smem_seg > (size_t)prop.sharedMemPerBlockOptin) {
