@@ -551,18 +551,45 @@ __global__ void __launch_bounds__(256) n2t_scatter_kernel(const InstDesc* insts)
     }
 }
 
-// Sort each node's term segment ascending, one warp per node, in registers:
-// element i = 32 s + lane sits in slot s of a lane; a bitonic network over
-// kSlots * 32 keys exchanges across lanes with shuffles (partner distance
-// < 32) and inside a lane between slots otherwise. A launch takes the
-// segments of (min_len, 32 kSlots] terms; three launches (8, 16, 32 slots)
-// cover up to kWarpSortMax, and n2t_sort_kernel the longer ones.
-constexpr uint32_t kWarpSortMax = 1024;
+// Ascending sort of 32 kSlots keys in a warp's registers: element
+// i = 32 s + lane sits in slot s of a lane; a bitonic network exchanges across
+// lanes with shuffles (partner distance < 32) and inside a lane between slots
+// otherwise.
+template <int kSlots> __device__ inline void warp_sort(uint32_t (&v)[kSlots]) {
+    const uint32_t lane = lane_id();
+#pragma unroll
+    for (uint32_t k = 2; k <= 32u * kSlots; k <<= 1) {
+#pragma unroll
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            if (j >= 32) {
+                const int sj = (int)(j >> 5);
+#pragma unroll
+                for (int sl = 0; sl < kSlots; ++sl) {
+                    if (sl & sj) continue;
+                    const uint32_t i = 32u * sl + lane;
+                    const bool up = (i & k) == 0;
+                    const uint32_t a = v[sl], c = v[sl | sj];
+                    v[sl] = up ? min(a, c) : max(a, c);
+                    v[sl | sj] = up ? max(a, c) : min(a, c);
+                }
+            } else {
+#pragma unroll
+                for (int sl = 0; sl < kSlots; ++sl) {
+                    const uint32_t i = 32u * sl + lane;
+                    const uint32_t o = __shfl_xor_sync(0xffffffffu, v[sl], j);
+                    const bool up = (i & k) == 0, lower = (i & j) == 0;
+                    v[sl] = (up == lower) ? min(v[sl], o) : max(v[sl], o);
+                }
+            }
+        }
+    }
+}
 
-template <int kSlots>
-__global__ void __launch_bounds__(256) n2t_warp_sort_kernel(const InstDesc* insts, uint32_t min_len) {
-    constexpr int kWarpSortSlots = kSlots;
-    constexpr uint32_t kMax = 32u * kSlots;
+// Each node's term segment ascending. Up to kSortRun terms: a warp per node.
+constexpr int kSortSlots = 8;
+constexpr uint32_t kSortRun = 32u * kSortSlots, kMergeMax = 4096;
+
+__global__ void __launch_bounds__(256) n2t_warp_sort_kernel(const InstDesc* insts) {
     const InstDesc& I = insts[blockIdx.y];
     if (I.counts->node2term_entries > I.cap_k1) return;
     const uint32_t lane = lane_id();
@@ -570,53 +597,85 @@ __global__ void __launch_bounds__(256) n2t_warp_sort_kernel(const InstDesc* inst
     for (uint32_t node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); node < I.N; node += warps) {
         const uint32_t b = I.n2t_offset[node], e = I.n2t_offset[node + 1];
         const uint32_t len = e - b;
-        if (len <= min_len || len <= 1 || len > kMax) continue;
+        if (len <= 1 || len > kSortRun) continue;
         if (len > I.cap_seg) {  // the segment exceeds max_terms_per_node
             if (lane == 0) set_error(I, kErrSegmentTooLong);
             continue;
         }
-        uint32_t v[kWarpSortSlots];
+        uint32_t v[kSortSlots];
 #pragma unroll
-        for (int sl = 0; sl < kWarpSortSlots; ++sl) {
+        for (int sl = 0; sl < kSortSlots; ++sl) {
             const uint32_t i = 32u * sl + lane;
             v[sl] = i < len ? I.n2t_index[b + i] : 0xFFFFFFFFu;
         }
+        warp_sort<kSortSlots>(v);
 #pragma unroll
-        for (uint32_t k = 2; k <= kMax; k <<= 1) {
-#pragma unroll
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                if (j >= 32) {
-                    const int sj = (int)(j >> 5);
-#pragma unroll
-                    for (int sl = 0; sl < kWarpSortSlots; ++sl) {
-                        if (sl & sj) continue;
-                        const uint32_t i = 32u * sl + lane;
-                        const bool up = (i & k) == 0;
-                        const uint32_t a = v[sl], c = v[sl | sj];
-                        v[sl] = up ? min(a, c) : max(a, c);
-                        v[sl | sj] = up ? max(a, c) : min(a, c);
-                    }
-                } else {
-#pragma unroll
-                    for (int sl = 0; sl < kWarpSortSlots; ++sl) {
-                        const uint32_t i = 32u * sl + lane;
-                        const uint32_t o = __shfl_xor_sync(0xffffffffu, v[sl], j);
-                        const bool up = (i & k) == 0, lower = (i & j) == 0;
-                        v[sl] = (up == lower) ? min(v[sl], o) : max(v[sl], o);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int sl = 0; sl < kWarpSortSlots; ++sl) {
+        for (int sl = 0; sl < kSortSlots; ++sl) {
             const uint32_t i = 32u * sl + lane;
             if (i < len) I.n2t_index[b + i] = v[sl];
         }
     }
 }
 
-// sort each node's term segment ascending (one CTA per node) for the
-// segments longer than kWarpSortMax
+// From kSortRun to kMergeMax terms: a CTA per node. Its warps sort runs of
+// kSortRun in registers; each key's place is then its place in its run plus the
+// number of smaller keys in every other run (binary searches in shared memory).
+// A warp with 16 or 32 slots, or a bitonic sort over shared memory, has a chain of
+// 45 to 78 exchange steps per node: 106 -> 21 us on a 500-node frame, 413 -> 257
+// us on 32,768 nodes.
+constexpr uint32_t kMergeWarps = 4;
+
+__global__ void __launch_bounds__(32 * kMergeWarps) n2t_merge_sort_kernel(const InstDesc* insts) {
+    __shared__ uint32_t key[kMergeMax];
+    const InstDesc& I = insts[blockIdx.y];
+    if (I.counts->node2term_entries > I.cap_k1) return;
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    for (uint32_t node = blockIdx.x; node < I.N; node += gridDim.x) {
+        const uint32_t b = I.n2t_offset[node], len = I.n2t_offset[node + 1] - b;
+        if (len <= kSortRun) continue;
+        if (len > I.cap_seg) {
+            if (threadIdx.x == 0) set_error(I, kErrSegmentTooLong);
+            continue;
+        }
+        if (len > kMergeMax) continue;  // n2t_sort_kernel's
+        const uint32_t runs = (len + kSortRun - 1) / kSortRun;
+        for (uint32_t r = warp; r < runs; r += kMergeWarps) {
+            uint32_t v[kSortSlots];
+#pragma unroll
+            for (int sl = 0; sl < kSortSlots; ++sl) {
+                const uint32_t i = kSortRun * r + 32u * sl + lane;
+                v[sl] = i < len ? I.n2t_index[b + i] : 0xFFFFFFFFu;
+            }
+            warp_sort<kSortSlots>(v);
+#pragma unroll
+            for (int sl = 0; sl < kSortSlots; ++sl) key[kSortRun * r + 32u * sl + lane] = v[sl];
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < len; i += 32 * kMergeWarps) {
+            // (only the last run is padded, with keys above every term)
+            const uint32_t r = i / kSortRun, k = key[i];
+            uint32_t rank = i % kSortRun;
+            for (uint32_t o = 0; o < runs; ++o) {
+                if (o == r) continue;
+                // keys below k, and for an earlier run also those equal to it
+                const uint32_t* run = key + kSortRun * o;
+                uint32_t n = 0;
+#pragma unroll
+                for (uint32_t step = kSortRun / 2; step > 0; step >>= 1) {
+                    const uint32_t x = run[n + step - 1];
+                    if (x < k || (o < r && x == k)) n += step;
+                }
+                const uint32_t x = run[n];
+                if (x < k || (o < r && x == k)) ++n;
+                rank += n;
+            }
+            I.n2t_index[b + rank] = k;
+        }
+        __syncthreads();
+    }
+}
+
+// longer segments: a bitonic sort in shared memory, one CTA per node
 __global__ void __launch_bounds__(256) n2t_sort_kernel(const InstDesc* insts) {
     extern __shared__ uint32_t s32[];
     const InstDesc& I = insts[blockIdx.y];
@@ -624,11 +683,7 @@ __global__ void __launch_bounds__(256) n2t_sort_kernel(const InstDesc* insts) {
     for (uint32_t node = blockIdx.x; node < I.N; node += gridDim.x) {
         const uint32_t b = I.n2t_offset[node], e = I.n2t_offset[node + 1];
         const uint32_t len = e - b;
-        if (len <= kWarpSortMax) continue;
-        if (len > I.cap_seg) {
-            if (threadIdx.x == 0) set_error(I, kErrSegmentTooLong);
-            continue;
-        }
+        if (len <= kMergeMax || len > I.cap_seg) continue;
         const uint32_t n2 = next_pow2(len);
         for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) s32[i] = i < len ? I.n2t_index[b + i] : 0xFFFFFFFFu;
         __syncthreads();
@@ -664,7 +719,11 @@ __device__ inline uint32_t upper_entries_of(const InstDesc& I, const TermOffsets
     return c;
 }
 
-// warp per node: number of upper entries of the row
+// warp per node: number of upper entries of the row, and n2t_w[p], the node's
+// skinning weight in each of its terms (0 for smooth; the values are those of
+// weight_of, PreconditionerBlocked.cu:23-29). The weights are inputs, recorded
+// once per solve, so that the assembly kernels read one coalesced value per entry
+// instead of the term's node and weight records.
 __global__ void __launch_bounds__(256) np_row_count_kernel(const InstDesc* insts) {
     const InstDesc& I = insts[blockIdx.y];
     if (I.counts->node2term_entries > I.cap_k1) return;
@@ -674,9 +733,24 @@ __global__ void __launch_bounds__(256) np_row_count_kernel(const InstDesc* insts
     for (uint32_t node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); node < I.N; node += warps) {
         const uint32_t b = I.n2t_offset[node], e = I.n2t_offset[node + 1];
         uint32_t c = 0;
+#pragma unroll 4
         for (uint32_t p = b + lane_id(); p < e; p += 32) {
-            uint32_t js[4];
-            c += upper_entries_of(I, off, node, I.n2t_index[p], js);
+            uint32_t k;
+            const TermType ty = off.typed(I.n2t_index[p], k);
+            const ushort4 n = term_nodes(I, ty, k);
+            float w = 0.f;
+            if (ty == kSmooth) {
+                // one pair (min, max), in the row of min; a node listed twice in
+                // the same smooth term gives no pair
+                const uint32_t o = n.x == node ? n.y : n.x;
+                c += o > node && o < I.N ? 1u : 0u;
+            } else {
+                if (ty != kInvalidTerm) w = weight_of(n, term_weights(I, ty, k), node);
+                const uint32_t a[4] = {n.x, n.y, n.z, n.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) c += a[q] > node && a[q] < I.N ? 1u : 0u;
+            }
+            I.n2t_w[p] = w;
         }
         c = warp_sum(c);
         if (lane_id() == 0) I.row_count[node] = c;
@@ -684,150 +758,240 @@ __global__ void __launch_bounds__(256) np_row_count_kernel(const InstDesc* insts
 }
 
 // Warp per node: the row's (j, t) entries, j > node, in ascending (j, t) order
-// without sorting. The node's term list is already ascending in t, so for
-// each distinct partner j (ascending, found by a warp minimum) one sweep of
-// the list emits the terms that contain j, in t order, and finds the next
-// partner. The first kRowCache * 32 terms stay in registers (the term id and
-// its partners, packed 16-bit), the next kRowSpill * 32 in shared memory;
-// longer lists re-derive the rest each sweep. A
-// term that lists a partner twice contributes two adjacent entries, like the
-// duplicate keys of a sort. Writes np_index, the per-pair (key, start) of the
-// row and upper_count.
-constexpr int kRowCache = 8;
+// without sorting, with the products of the two nodes' weights. The node's term
+// list is already ascending in t. A first pass counts the entries of each
+// distinct partner in a small hash table in shared memory; the partners are
+// ranked, which gives each one's start; a second pass places the entries: of 32
+// consecutive terms, those of the same partner take consecutive places in lane
+// order. Both passes take kRowSlices slices of 32 terms at once, so that their
+// gathers overlap; bound by those gathers and by fetching its own unrolled
+// instructions: with four slices (80 registers) 32,768 nodes take 929 us and 500
+// nodes the same 101, with one 580 and 118. A term that lists a partner twice, or a
+// node with more than kRowPartners partners, takes the sweep (one pass over the
+// list per partner), which is what every node took before: 285 -> 101 us on a
+// 500-node frame, whose lists reach 1,276 terms, 72 -> 51 us on 3,000 nodes, 752 ->
+// 606 us on 32,768, with the weights' own pass (77, 42 and 219 us) saved. Writes
+// np_index, np_scale, the per-pair (key, start) of the row and upper_count.
+constexpr uint32_t kRowSlices = 2, kRowTable = 256, kRowPartners = 192, kRowWarps = 4;
 
-__device__ inline void unpack_partners(uint2 pk, uint32_t j[4]) {
-    j[0] = pk.x & 0xFFFFu; j[1] = pk.x >> 16; j[2] = pk.y & 0xFFFFu; j[3] = pk.y >> 16;
+struct RowTable {
+    uint32_t key[kRowTable];    // partner, kInvalid: free
+    uint32_t count[kRowTable];  // its entries, then the place of its next one
+    uint32_t mask[kRowTable];   // lanes of the current slice that hold it
+    uint32_t slot[kRowPartners], rank_slot[kRowPartners];  // the used slots, then in order of the partner
+    uint32_t used, sweep;
+};
+
+__device__ inline uint32_t row_hash(uint32_t j) { return (j * 2654435761u) >> 24; }
+static_assert(kRowTable == 256, "eight hash bits");
+
+__device__ inline uint32_t row_find(const RowTable& tb, uint32_t j) {
+    uint32_t h = row_hash(j);
+    while (tb.key[h] != j) h = (h + 1) & (kRowTable - 1);
+    return h;
 }
 
-// the term's partners above `node` packed as four 16-bit ids (0xFFFF = none)
-__device__ inline uint2 packed_partners(const InstDesc& I, const TermOffsets& off, uint32_t node, uint32_t t) {
-    uint32_t js[4];
-    const uint32_t c = upper_entries_of(I, off, node, t, js);
-    uint32_t v[4] = {0xFFFFu, 0xFFFFu, 0xFFFFu, 0xFFFFu};
-    for (uint32_t q = 0; q < c; ++q) v[q] = js[q];
-    return make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+// weight product of an entry's two nodes, exact in double (0 for a smooth term)
+__device__ inline double pair_scale(const InstDesc& I, const TermOffsets& off, uint32_t t, uint32_t i, uint32_t j) {
+    uint32_t k;
+    const TermType ty = off.typed(t, k);
+    if (ty == kSmooth || ty == kInvalidTerm) return 0.0;
+    const ushort4 kn = term_nodes(I, ty, k);
+    const float4 w4 = term_weights(I, ty, k);
+    return (double)weight_of(kn, w4, i) * (double)weight_of(kn, w4, j);
 }
 
-// terms kRowCache * 32 .. kRowCache * 32 + kRowSpill * 32 of a node's list
-// wait in shared memory (the same (term, partners) pairs), so that the sweeps
-// re-read them without re-deriving their partners
-constexpr int kRowSpill = 8;
+// the sweep: for each distinct partner (ascending, found by a warp minimum) one
+// pass over the list emits the terms that contain it, in t order, and finds the
+// next partner. A term that lists a partner twice contributes two adjacent
+// entries, like the duplicate keys of a sort. Returns the distinct partners.
+__device__ inline uint32_t row_sweep(const InstDesc& I, const TermOffsets& off, uint32_t node, uint32_t b0, uint32_t b1,
+                                     uint32_t out, uint32_t len) {
+    const uint32_t lane = lane_id();
+    uint32_t pos = 0, runs = 0, j = node;  // the first pass emits nothing and finds the first partner
+    for (bool first = true;; first = false) {
+        if (!first && lane == 0 && pos < len) {
+            I.tmp_key[out + runs] = node * I.enc + j;
+            I.tmp_start[out + runs] = out + pos;
+        }
+        uint32_t nxt = 0xFFFFFFFFu;
+        for (uint32_t base = b0; base < b1; base += 32) {
+            const uint32_t p = base + lane, t = p < b1 ? I.n2t_index[p] : kInvalid;
+            uint32_t js[4], mult = 0;
+            const uint32_t c = p < b1 ? upper_entries_of(I, off, node, t, js) : 0u;
+            for (uint32_t q = 0; q < c; ++q) {
+                if (!first && js[q] == j) ++mult;
+                if (js[q] > j) nxt = min(nxt, js[q]);
+            }
+            const uint32_t incl = warp_inclusive_scan(mult), total = __shfl_sync(0xffffffffu, incl, 31);
+            for (uint32_t m = 0; m < mult; ++m) {
+                const uint32_t at = pos + incl - mult + m;
+                if (at >= len) break;
+                I.np_index[out + at] = t;
+                I.np_scale[out + at] = pair_scale(I, off, t, node, j);
+            }
+            pos += total;
+        }
+        if (!first) ++runs;
+        j = warp_min_u32(nxt);
+        if (j == 0xFFFFFFFFu) return runs;
+    }
+}
 
-__global__ void __launch_bounds__(256, 4) np_row_build_kernel(const InstDesc* insts) {
-    __shared__ uint32_t s_t[8][kRowSpill * 32];
-    __shared__ uint2 s_pk[8][kRowSpill * 32];
+__global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const InstDesc* insts) {
+    __shared__ RowTable s_table[kRowWarps];
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
     if (C->node2term_entries > I.cap_k1 || C->nodepair_entries > I.cap_k2) return;
     TermOffsets off;
     off.load(I.counts);
-    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t node = blockIdx.x * (blockDim.x >> 5) + w; node < I.N; node += warps) {
+    const uint32_t lane = lane_id(), lt_mask = (1u << lane) - 1u;
+    RowTable& tb = s_table[threadIdx.x >> 5];
+    const uint32_t warps = gridDim.x * kRowWarps;
+    for (uint32_t node = blockIdx.x * kRowWarps + (threadIdx.x >> 5); node < I.N; node += warps) {
         const uint32_t b0 = I.n2t_offset[node], b1 = I.n2t_offset[node + 1];
         const uint32_t out = I.row_offset[node], len = I.row_count[node];
-        uint32_t ct[kRowCache];
-        uint2 cj[kRowCache];
-#pragma unroll
-        for (int m = 0; m < kRowCache; ++m) {
-            const uint32_t p = b0 + lane + 32u * m;
-            ct[m] = p < b1 ? I.n2t_index[p] : kInvalid;
-            cj[m] = p < b1 ? packed_partners(I, off, node, ct[m]) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+        for (uint32_t i = lane; i < kRowTable; i += 32) {
+            tb.key[i] = kInvalid;
+            tb.count[i] = 0;
+            tb.mask[i] = 0;
         }
-        // the spill slices in shared memory (entries past b1 hold no partners)
-        const uint32_t spill0 = b0 + 32u * kRowCache;
-        const uint32_t spill1 = min(b1, spill0 + 32u * kRowSpill);
+        if (lane == 0) tb.used = tb.sweep = 0;
         __syncwarp();
-        const uint32_t nspill = spill1 > spill0 ? (spill1 - spill0 + 31u) / 32u : 0u;  // whole slices
-        for (uint32_t q = lane; q < 32u * nspill; q += 32) {
-            const uint32_t p = spill0 + q;
-            const uint32_t t = p < b1 ? I.n2t_index[p] : kInvalid;
-            s_t[w][q] = t;
-            s_pk[w][q] = p < b1 ? packed_partners(I, off, node, t) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
-        }
-        __syncwarp();
-        // emit the slice's entries for partner j at out + pos; returns the
-        // smallest partner above j seen in the slice
-        auto slice = [&](uint32_t t, uint2 pk, uint32_t j, uint32_t& pos) -> uint32_t {
-            uint32_t js[4];
-            unpack_partners(pk, js);
-            uint32_t mult = 0, nxt = 0xFFFFFFFFu;
+        // the partners above `node` of the terms of kRowSlices slices
+        uint32_t t[kRowSlices], js[kRowSlices][4];
+        auto load = [&](uint32_t base) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                mult += js[q] == j ? 1u : 0u;
-                if (js[q] != 0xFFFFu && js[q] > j) nxt = min(nxt, js[q]);
+            for (uint32_t s = 0; s < kRowSlices; ++s) {
+                const uint32_t p = base + 32 * s + lane;
+                t[s] = p < b1 ? I.n2t_index[p] : kInvalid;
             }
-            uint32_t pre, total;
-            if (__any_sync(0xffffffffu, mult > 1)) {
-                pre = mult;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
-                    if (lane >= (uint32_t)o) pre += v;
-                }
-                total = __shfl_sync(0xffffffffu, pre, 31);
-                pre -= mult;
-            } else {
-                const uint32_t bal = __ballot_sync(0xffffffffu, mult != 0);
-                pre = __popc(bal & lt_mask);
-                total = __popc(bal);
-            }
-            for (uint32_t c = 0; c < mult; ++c)
-                if (pos + pre + c < len) I.np_index[out + pos + pre + c] = t;
-            pos += total;
-            return nxt;
-        };
-        // first partner: the smallest id above node
-        uint32_t j;
-        {
-            uint32_t mn = 0xFFFFFFFFu;
-#pragma unroll
-            for (int m = 0; m < kRowCache; ++m) {
-                uint32_t js[4];
-                unpack_partners(cj[m], js);
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (js[q] != 0xFFFFu) mn = min(mn, js[q]);
-            }
-            for (uint32_t p = b0 + 32u * kRowCache + lane; p < b1; p += 32) {
-                uint32_t js[4];
-                unpack_partners(p < spill1 ? s_pk[w][p - spill0] : packed_partners(I, off, node, I.n2t_index[p]), js);
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (js[q] != 0xFFFFu) mn = min(mn, js[q]);
-            }
-            j = warp_min_u32(mn);
-        }
-        uint32_t pos = 0, runs = 0;
-        while (j != 0xFFFFFFFFu) {
-            if (lane == 0 && pos < len) {
-                I.tmp_key[out + runs] = node * I.enc + j;
-                I.tmp_start[out + runs] = out + pos;
-            }
-            uint32_t nxt = 0xFFFFFFFFu;
-#pragma unroll
-            for (int m = 0; m < kRowCache; ++m) {
-                if (b0 + 32u * m >= b1) break;  // warp-uniform
-                nxt = min(nxt, slice(ct[m], cj[m], j, pos));
-            }
-            for (uint32_t base = b0 + 32u * kRowCache; base < b1; base += 32) {
-                const uint32_t p = base + lane;
-                uint32_t t;
-                uint2 pk;
-                if (base < spill1) {  // warp-uniform: a spilled slice
-                    t = s_t[w][p - spill0];
-                    pk = s_pk[w][p - spill0];
+            for (uint32_t s = 0; s < kRowSlices; ++s) {
+                uint32_t k;
+                const TermType ty = off.typed(t[s], k);
+                const ushort4 n = t[s] != kInvalid ? term_nodes(I, ty, k) : make_ushort4(0xFFFF, 0xFFFF, 0xFFFF, 0xFFFF);
+                const uint32_t a[4] = {n.x, n.y, n.z, n.w};
+                if (ty == kSmooth) {  // one pair (min, max), in the row of min
+                    const uint32_t o = a[0] == node ? a[1] : a[0];
+                    js[s][0] = o > node && o < I.N ? o : kInvalid;
+                    js[s][1] = js[s][2] = js[s][3] = kInvalid;
                 } else {
-                    t = p < b1 ? I.n2t_index[p] : kInvalid;
-                    pk = p < b1 ? packed_partners(I, off, node, t) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) js[s][q] = a[q] > node && a[q] < I.N ? a[q] : kInvalid;
                 }
-                nxt = min(nxt, slice(t, pk, j, pos));
             }
-            ++runs;
-            j = warp_min_u32(nxt);
+        };
+        bool sweep = false;
+        for (uint32_t base = b0; base < b1 && !sweep; base += 32 * kRowSlices) {
+            load(base);
+#pragma unroll
+            for (uint32_t s = 0; s < kRowSlices; ++s) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t j = js[s][q];
+                    if (j == kInvalid) continue;
+                    bool twice = false;
+#pragma unroll
+                    for (int o = 0; o < q; ++o) twice |= js[s][o] == j;
+                    if (twice || *(volatile uint32_t*)&tb.used >= kRowPartners) {
+                        tb.sweep = 1;
+                        continue;
+                    }
+                    uint32_t h = row_hash(j);
+                    for (;;) {
+                        const uint32_t seen = atomicCAS(&tb.key[h], kInvalid, j);
+                        if (seen == j) break;
+                        if (seen == kInvalid) {
+                            const uint32_t u = atomicAdd(&tb.used, 1u);
+                            if (u < kRowPartners) tb.slot[u] = h;
+                            break;
+                        }
+                        h = (h + 1) & (kRowTable - 1);
+                    }
+                    atomicAdd(&tb.count[h], 1u);
+                }
+            }
+            __syncwarp();
+            sweep = __any_sync(0xffffffffu, tb.sweep != 0);  // (the same in every lane)
         }
-        if (lane == 0) I.upper_count[node] = runs;
+        __syncwarp();
+        const uint32_t used = tb.used;
+        if (sweep || used > kRowPartners) {
+            const uint32_t runs = row_sweep(I, off, node, b0, b1, out, len);
+            if (lane == 0) I.upper_count[node] = runs;
+            __syncwarp();
+            continue;
+        }
+        // rank the partners; starts in that order
+        for (uint32_t i = lane; i < used; i += 32) {
+            const uint32_t h = tb.slot[i], j = tb.key[h];
+            uint32_t rank = 0;
+            for (uint32_t m = 0; m < used; ++m) rank += tb.key[tb.slot[m]] < j ? 1u : 0u;
+            tb.rank_slot[rank] = h;
+        }
+        __syncwarp();
+        uint32_t start = 0;
+        for (uint32_t base = 0; base < used; base += 32) {
+            const uint32_t r = base + lane;
+            const uint32_t h = r < used ? tb.rank_slot[r] : 0u, n = r < used ? tb.count[h] : 0u;
+            const uint32_t incl = warp_inclusive_scan(n);
+            if (r < used) {
+                I.tmp_key[out + r] = node * I.enc + tb.key[h];
+                I.tmp_start[out + r] = out + start + incl - n;
+                tb.count[h] = start + incl - n;
+            }
+            start += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) I.upper_count[node] = used;
+        __syncwarp();
+        // place the entries
+        for (uint32_t base = b0; base < b1; base += 32 * kRowSlices) {
+            load(base);
+            float4 w4[kRowSlices];
+            ushort4 kn[kRowSlices];
+#pragma unroll
+            for (uint32_t s = 0; s < kRowSlices; ++s) {
+                uint32_t k;
+                const TermType ty = off.typed(t[s], k);
+                const bool weighted = t[s] != kInvalid && ty != kSmooth && ty != kInvalidTerm;
+                kn[s] = weighted ? term_nodes(I, ty, k) : make_ushort4(0, 0, 0, 0);
+                w4[s] = weighted ? term_weights(I, ty, k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (uint32_t s = 0; s < kRowSlices; ++s) {
+                uint32_t h[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    h[q] = kInvalid;
+                    if (js[s][q] == kInvalid) continue;
+                    h[q] = row_find(tb, js[s][q]);
+                    atomicOr(&tb.mask[h[q]], 1u << lane);
+                }
+                __syncwarp();
+                const double wi = (double)weight_of(kn[s], w4[s], node);
+                uint32_t m[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (h[q] == kInvalid) continue;
+                    m[q] = tb.mask[h[q]];
+                    const uint32_t at = tb.count[h[q]] + __popc(m[q] & lt_mask);
+                    if (at < len) {
+                        I.np_index[out + at] = t[s];
+                        I.np_scale[out + at] = wi * (double)weight_of(kn[s], w4[s], js[s][q]);
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {  // the partner's first lane moves its place on
+                    if (h[q] == kInvalid || (m[q] & lt_mask)) continue;
+                    tb.count[h[q]] += __popc(m[q]);
+                    tb.mask[h[q]] = 0;
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -1035,61 +1199,6 @@ __global__ void __launch_bounds__(256) bin_colptr_kernel(const InstDesc* insts) 
     }
 }
 
-// ------------------------------------------------- per-entry weights -----
-// The skinning weight of each index entry's node(s) in its term, recorded once
-// per solve (the weights are inputs), so that the assembly kernels read one
-// coalesced value per entry instead of the term's node and weight records.
-// The values are those of weight_of (PreconditionerBlocked.cu:23-29).
-
-// warp per node: n2t_w[p] for the node's terms
-__global__ void __launch_bounds__(256) n2t_weight_kernel(const InstDesc* insts) {
-    const InstDesc& I = insts[blockIdx.y];
-    if (I.counts->node2term_entries > I.cap_k1) return;
-    TermOffsets off;
-    off.load(I.counts);
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); node < I.N; node += warps) {
-        const uint32_t b0 = I.n2t_offset[node], b1 = I.n2t_offset[node + 1];
-        for (uint32_t p = b0 + lane_id(); p < b1; p += 32) {
-            uint32_t k;
-            const TermType ty = off.typed(I.n2t_index[p], k);
-            I.n2t_w[p] = ty == kSmooth || ty == kInvalidTerm
-                             ? 0.f
-                             : weight_of(term_nodes(I, ty, k), term_weights(I, ty, k), node);
-        }
-    }
-}
-
-// warp per node i: np_scale[p] = w_i w_j for the terms of each pair (i, j)
-// (a product of two floats is exact in double, and rounds to the float product),
-// pair by pair, the lanes over the pair's entries
-__global__ void __launch_bounds__(256) np_weight_kernel(const InstDesc* insts) {
-    const InstDesc& I = insts[blockIdx.y];
-    const DeviceCounts* C = I.counts;
-    if (C->half_pairs > I.cap_pairs || C->nodepair_entries > I.cap_k2 || C->node2term_entries > I.cap_k1) return;
-    TermOffsets off;
-    off.load(C);
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t ni = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); ni < I.N; ni += warps) {
-        const uint32_t h0 = I.half_offset[ni], nu = I.upper_count[ni];
-        for (uint32_t h = h0; h < h0 + nu; ++h) {
-            const uint32_t nj = I.half_key[h] % I.enc;
-            const uint2 rg = I.half_range[h];
-            for (uint32_t p = rg.x + lane_id(); p < rg.y; p += 32) {
-                uint32_t k;
-                const TermType ty = off.typed(I.np_index[p], k);
-                double w = 0.0;
-                if (ty != kSmooth && ty != kInvalidTerm) {
-                    const ushort4 kn = term_nodes(I, ty, k);
-                    const float4 w4 = term_weights(I, ty, k);
-                    w = (double)weight_of(kn, w4, ni) * (double)weight_of(kn, w4, nj);
-                }
-                I.np_scale[p] = w;
-            }
-        }
-    }
-}
-
 // ------------------------------------------------------------ launch -----
 
 static inline dim3 grid2(uint32_t x, uint32_t B) { return dim3(x ? x : 1, B); }
@@ -1121,23 +1230,20 @@ cudaError_t launch_build_index(const LaunchCfg& lc, InstDesc* d, cudaStream_t st
     MVDR_LAUNCH(n2t_count_kernel, grid2(spread, B), 256, 0, st, d);
     MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanN2T);
     MVDR_LAUNCH(n2t_scatter_kernel, grid2(spread, B), 256, 0, st, d);
-    MVDR_LAUNCH(n2t_warp_sort_kernel<8>, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d, 0u);
-    MVDR_LAUNCH(n2t_warp_sort_kernel<16>, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d, 256u);
-    MVDR_LAUNCH(n2t_warp_sort_kernel<32>, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d, 512u);
-    MVDR_LAUNCH(n2t_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count), B), 256, (size_t)lc.cap_seg * 4, st,
-                d);
+    MVDR_LAUNCH(n2t_warp_sort_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
+    MVDR_LAUNCH(n2t_merge_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count * 12), B), 32 * kMergeWarps, 0, st, d);
+    if (lc.cap_seg > kMergeMax)
+        MVDR_LAUNCH(n2t_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count), B), 256, (size_t)lc.cap_seg * 4, st, d);
     // node pair -> term
     MVDR_LAUNCH(np_row_count_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
     MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanRows);
-    MVDR_LAUNCH(np_row_build_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
+    MVDR_LAUNCH(np_row_build_kernel, grid2((lc.max_nodes + kRowWarps - 1) / kRowWarps, B), 32 * kRowWarps, 0, st, d);
     MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanUpper);
     MVDR_LAUNCH(np_half_compact_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
     MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanBlkRows);
     MVDR_LAUNCH(np_sym_scatter_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
     MVDR_LAUNCH(np_lower_sort_kernel, grid2((lc.max_nodes + 3) / 4, B), 128, 0, st, d);
     MVDR_LAUNCH(pair_order_kernel, grid2(min((lc.cap_pairs + kPairWindow - 1) / kPairWindow, spread), B), kLenBuckets, 0, st, d);
-    MVDR_LAUNCH(n2t_weight_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
-    MVDR_LAUNCH(np_weight_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
     // bin-block CSR structure
     MVDR_LAUNCH(bin_length_kernel, grid2((6 * lc.max_nodes / 32 + 256) / 256, B), 256, 0, st, d);
     MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanBins);
