@@ -1,0 +1,36 @@
+"""Node errors at the edges of the kernel's pixel tiles, and with skinning weights
+that its summed form does not take (negative, above 2^18): equal to the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from multiviewdynrecon_b200 import abi, synth
+from multiviewdynrecon_b200.solver import NonRigidSolver
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("width,height,weights", [(97, 65, None), (64, 72, None), (129, 57, "large"), (65, 67, "mixed")])
+def test_node_error_equals_the_oracle(oracle_mod, width, height, weights):
+    scene = synth.sphere_single_view(seed=4, num_nodes=40, width=width, height=height)
+    rng = np.random.default_rng(6)
+    w = rng.uniform(0.05, 0.4, scene.surfel_knn_weight.shape).astype(np.float32)
+    if weights == "large":
+        w *= np.float32(1 << 22)
+    elif weights == "mixed":
+        some = rng.random(len(w)) < 0.02
+        w[some] *= np.float32(-3e6)
+    scene.surfel_knn_weight[:] = w
+    # (a node twice among a surfel's four is added twice)
+    scene.surfel_knn[::7, 3] = scene.surfel_knn[::7, 0]
+    solver = NonRigidSolver(abi.make_config(scene))
+    solver.set_solver_input(scene)
+    got = solver.compute_alignment_error_on_nodes(maps=True)
+    torch.cuda.synchronize()
+    want = oracle_mod.node_error(scene, scene.node_se3, maps=True)
+    for k in ("accumulated_error", "accumulated_weight", "united_error", "large_error_mark"):
+        assert np.array_equal(got[k].cpu().numpy().astype(want[k].dtype), want[k], equal_nan=True), k
+    for k in ("alignment_error_map", "node_error_map"):
+        assert np.array_equal(got[k][0].cpu().numpy(), want[k][0], equal_nan=True), k
+    assert (want["accumulated_error"] != 0).sum() > 10
+    solver.close()
