@@ -12,6 +12,40 @@ namespace mvdr {
         count_launch();                                           \
     } while (0)
 
+// Launches the kernel so that it may start while the kernel before it in the stream
+// still runs (programmatic dependent launch): its blocks take their places and wait
+// in chain_wait(), its first statement, until that kernel has finished and its
+// writes are visible.
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+    count_launch();
+}
+
+// `chained` (a host value): launch_chained, else MVDR_LAUNCH
+#define MVDR_LAUNCH_IF_CHAINED(chained, kernel, grid, block, smem, stream, ...)            \
+    do {                                                                                   \
+        if (chained) launch_chained(kernel, (grid), (block), (smem), (stream), __VA_ARGS__); \
+        else MVDR_LAUNCH(kernel, grid, block, smem, stream, __VA_ARGS__);                  \
+    } while (0)
+
+// The first statement of every kernel that is launched chained: lets the next kernel
+// take its place, then waits for the one before (at once where neither is chained).
+__device__ inline void chain_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ inline uint32_t lane_id() { return threadIdx.x & 31u; }
 
 template <class T> __device__ inline T warp_sum(T v) {
