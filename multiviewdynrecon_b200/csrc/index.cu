@@ -24,6 +24,7 @@ constexpr uint32_t kChunk = kChunkPixels;
 // below num_nodes and surfel ids below num_surfels; otherwise the instance is
 // flagged and every kernel that would index with them skips its work.
 __global__ void __launch_bounds__(256) input_check_kernel(const InstDesc* insts, uint32_t width, uint32_t height) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -96,6 +97,7 @@ struct ForegroundPred {
 template <class Pred>
 __global__ void __launch_bounds__(256, 6) compact_count_kernel(const InstDesc* insts, uint32_t width, uint32_t height,
                                                             uint32_t cpv) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const uint32_t view = blockIdx.x / cpv, c = blockIdx.x % cpv;
     uint32_t cnt = 0;
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(256, 6) compact_count_kernel(const InstDesc* i
 // exclusive scan of the chunk counts; per-view totals; capacity check
 __global__ void __launch_bounds__(1024) compact_scan_kernel(const InstDesc* insts, uint32_t cpv, uint32_t max_views,
                                                             int foreground) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     DeviceCounts* C = I.counts;
     // per-view totals before the scan
@@ -154,6 +157,7 @@ __global__ void __launch_bounds__(1024) compact_scan_kernel(const InstDesc* inst
 template <class Pred>
 __global__ void __launch_bounds__(256) compact_write_kernel(const InstDesc* insts, uint32_t width, uint32_t height,
                                                             uint32_t cpv, int foreground) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const uint32_t view = blockIdx.x / cpv, c = blockIdx.x % cpv;
     if (view >= I.num_views) return;
@@ -214,6 +218,7 @@ __device__ inline uint32_t sample_view(const InstDesc& I, ushort4 pix, uint32_t 
 // canonical vertex / normal of each compacted pixel in frame 0; constant over
 // the Gauss-Newton iterations, so computed once per index build
 __global__ void __launch_bounds__(256) prepare_pixels_kernel(const InstDesc* insts, bool mixed) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
     const uint32_t Td = C->dense_terms, Tf = C->foreground_terms;
@@ -302,6 +307,7 @@ __device__ inline float3 apply3_rn(const M34& m, float3 p) {
 
 // chooseValidPixelKernel: one thread per candidate pair
 __global__ void __launch_bounds__(256) feat_choose_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     if (!I.feat_select) return;
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -361,6 +367,7 @@ __global__ void __launch_bounds__(256) feat_choose_kernel(const InstDesc* insts)
 // 1024 threads per instance: an exclusive scan of the keep flags, then each
 // kept pair written at its prefix)
 __global__ void __launch_bounds__(1024) feat_compact_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     if (!I.feat_select) return;
     const uint32_t n = I.fp_offset[MVDR_MAX_VIEWS];
@@ -391,6 +398,7 @@ __global__ void __launch_bounds__(1024) feat_compact_kernel(const InstDesc* inst
 
 // size2offset (term_offset_types.h:44-64) on the device
 __global__ void term_offsets_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     if (threadIdx.x != 0) return;
     DeviceCounts* C = I.counts;
@@ -417,6 +425,7 @@ __global__ void term_offsets_kernel(const InstDesc* insts) {
 // hold the same node are merged (match_any) and one lane adds the group's
 // count: one atomic per distinct node and slot in the warp.
 __global__ void __launch_bounds__(256) n2t_count_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     if (bad_inputs(I)) return;
     TermOffsets off;
@@ -450,6 +459,7 @@ __global__ void __launch_bounds__(256) n2t_count_kernel(const InstDesc* insts) {
 enum ScanWhat : int { kScanN2T = 0, kScanRows = 1, kScanUpper = 2, kScanBlkRows = 3, kScanBins = 4 };
 
 __global__ void __launch_bounds__(1024) node_scan_kernel(const InstDesc* insts, int what) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     DeviceCounts* C = I.counts;
     __shared__ uint32_t total;
@@ -519,6 +529,7 @@ __global__ void __launch_bounds__(1024) node_scan_kernel(const InstDesc* insts, 
 // The same grouping: the group's first lane reserves the group's slots and
 // every lane takes its rank in the group (the sort that follows orders them).
 __global__ void __launch_bounds__(256) n2t_scatter_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     TermOffsets off;
     off.load(I.counts);
@@ -590,6 +601,7 @@ constexpr int kSortSlots = 8;
 constexpr uint32_t kSortRun = 32u * kSortSlots, kMergeMax = 4096;
 
 __global__ void __launch_bounds__(256) n2t_warp_sort_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     if (I.counts->node2term_entries > I.cap_k1) return;
     const uint32_t lane = lane_id();
@@ -626,6 +638,7 @@ __global__ void __launch_bounds__(256) n2t_warp_sort_kernel(const InstDesc* inst
 constexpr uint32_t kMergeWarps = 4;
 
 __global__ void __launch_bounds__(32 * kMergeWarps) n2t_merge_sort_kernel(const InstDesc* insts) {
+    chain_wait();
     __shared__ uint32_t key[kMergeMax];
     const InstDesc& I = insts[blockIdx.y];
     if (I.counts->node2term_entries > I.cap_k1) return;
@@ -677,6 +690,7 @@ __global__ void __launch_bounds__(32 * kMergeWarps) n2t_merge_sort_kernel(const 
 
 // longer segments: a bitonic sort in shared memory, one CTA per node
 __global__ void __launch_bounds__(256) n2t_sort_kernel(const InstDesc* insts) {
+    chain_wait();
     extern __shared__ uint32_t s32[];
     const InstDesc& I = insts[blockIdx.y];
     if (I.counts->node2term_entries > I.cap_k1) return;
@@ -725,6 +739,7 @@ __device__ inline uint32_t upper_entries_of(const InstDesc& I, const TermOffsets
 // once per solve, so that the assembly kernels read one coalesced value per entry
 // instead of the term's node and weight records.
 __global__ void __launch_bounds__(256) np_row_count_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     if (I.counts->node2term_entries > I.cap_k1) return;
     TermOffsets off;
@@ -839,6 +854,7 @@ __device__ inline uint32_t row_sweep(const InstDesc& I, const TermOffsets& off, 
 }
 
 __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const InstDesc* insts) {
+    chain_wait();
     __shared__ RowTable s_table[kRowWarps];
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
@@ -998,6 +1014,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const I
 // warp per node: copy the row's unique pairs to the compact half-pair arrays
 // and count the lower-triangle entries of each column
 __global__ void __launch_bounds__(256) np_half_compact_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
     if (C->half_pairs > I.cap_pairs || C->nodepair_entries > I.cap_k2 || C->node2term_entries > I.cap_k1) return;
@@ -1020,6 +1037,7 @@ __global__ void __launch_bounds__(256) np_half_compact_kernel(const InstDesc* in
 // warp per node: place the row's upper entries and scatter its pairs into the
 // lower part of each partner row (unordered there; sorted next)
 __global__ void __launch_bounds__(256) np_sym_scatter_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
     if (C->half_pairs > I.cap_pairs || C->nodepair_entries > I.cap_k2 || C->node2term_entries > I.cap_k1) return;
@@ -1055,6 +1073,7 @@ __global__ void __launch_bounds__(256) np_sym_scatter_kernel(const InstDesc* ins
 constexpr uint32_t kLenBuckets = 256;
 
 __global__ void __launch_bounds__(kLenBuckets) pair_order_kernel(const InstDesc* insts) {
+    chain_wait();
     constexpr uint32_t kPer = kPairWindow / kLenBuckets;
     __shared__ uint32_t count[kLenBuckets], warp_tot[kLenBuckets / 32], order[kPairWindow];
     const InstDesc& I = insts[blockIdx.y];
@@ -1100,6 +1119,7 @@ __global__ void __launch_bounds__(kLenBuckets) pair_order_kernel(const InstDesc*
 
 // warp per row: sort the lower part by key (keys are unique) by ranking
 __global__ void __launch_bounds__(128) np_lower_sort_kernel(const InstDesc* insts) {
+    chain_wait();
     constexpr uint32_t kMaxLower = 256;
     __shared__ uint32_t sk[4][kMaxLower];
     __shared__ uint2 sr[4][kMaxLower];
@@ -1154,6 +1174,7 @@ __global__ void __launch_bounds__(128) np_lower_sort_kernel(const InstDesc* inst
 // bin width is 6 x the longest block row (diagonal included) among the block
 // rows that the bin's 32 scalar rows touch
 __global__ void __launch_bounds__(256) bin_length_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const uint32_t nb = (6 * I.N + 31) / 32;
     if (blockIdx.x == 0 && threadIdx.x == 0) I.counts->num_bins = nb;
@@ -1171,6 +1192,7 @@ __global__ void __launch_bounds__(256) bin_length_kernel(const InstDesc* insts) 
 // computeBinBlockedCSRRowPtrKernel (NodePairRowColumnIndex.cu:122-132) and the
 // 0xFF fill of the column array (:273-281)
 __global__ void __launch_bounds__(256) bin_rowptr_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
     const uint32_t nb = C->num_bins;
@@ -1184,6 +1206,7 @@ __global__ void __launch_bounds__(256) bin_rowptr_kernel(const InstDesc* insts) 
 
 // computeBinBlockedCSRColPtrKernel (NodePairRowColumnIndex.cu:136-179)
 __global__ void __launch_bounds__(256) bin_colptr_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
     if (C->binblock_nnz > I.cap_bb || C->half_pairs > I.cap_pairs) return;
@@ -1211,44 +1234,45 @@ cudaError_t launch_build_index(const LaunchCfg& lc, InstDesc* d, cudaStream_t st
     const uint32_t B = lc.B;
     const uint32_t cpv = lc.chunks_per_view;
     const uint32_t spread = (uint32_t)lc.sm_count * 4;  // grid-stride kernels
+    const bool chain = chain_kernels(lc);
     MVDR_LAUNCH(input_check_kernel, grid2(spread, B), 256, 0, st, d, lc.width, lc.height);
     // dense pixels
-    MVDR_LAUNCH(compact_count_kernel<DensePred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv);
-    MVDR_LAUNCH(compact_scan_kernel, grid2(1, B), 1024, 0, st, d, cpv, lc.max_views, 0);
-    MVDR_LAUNCH(compact_write_kernel<DensePred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv, 0);
+    MVDR_LAUNCH_IF_CHAINED(chain, compact_count_kernel<DensePred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv);
+    MVDR_LAUNCH_IF_CHAINED(chain, compact_scan_kernel, grid2(1, B), 1024, 0, st, d, cpv, lc.max_views, 0);
+    MVDR_LAUNCH_IF_CHAINED(chain, compact_write_kernel<DensePred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv, 0);
     // foreground pixels (the predicate is false when the term is off)
-    MVDR_LAUNCH(compact_count_kernel<ForegroundPred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv);
-    MVDR_LAUNCH(compact_scan_kernel, grid2(1, B), 1024, 0, st, d, cpv, lc.max_views, 1);
-    MVDR_LAUNCH(compact_write_kernel<ForegroundPred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv, 1);
-    MVDR_LAUNCH(prepare_pixels_kernel, grid2(spread, B), 256, 0, st, d, lc.precision == MVDR_PRECISION_MIXED);
+    MVDR_LAUNCH_IF_CHAINED(chain, compact_count_kernel<ForegroundPred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv);
+    MVDR_LAUNCH_IF_CHAINED(chain, compact_scan_kernel, grid2(1, B), 1024, 0, st, d, cpv, lc.max_views, 1);
+    MVDR_LAUNCH_IF_CHAINED(chain, compact_write_kernel<ForegroundPred>, grid2(cpv * lc.max_views, B), 256, 0, st, d, lc.width, lc.height, cpv, 1);
+    MVDR_LAUNCH_IF_CHAINED(chain, prepare_pixels_kernel, grid2(spread, B), 256, 0, st, d, lc.precision == MVDR_PRECISION_MIXED);
     if (lc.max_tp) {
-        MVDR_LAUNCH(feat_choose_kernel, grid2((lc.max_tp + 255) / 256, B), 256, 0, st, d);
-        MVDR_LAUNCH(feat_compact_kernel, grid2(1, B), 1024, 0, st, d);
+        MVDR_LAUNCH_IF_CHAINED(chain, feat_choose_kernel, grid2((lc.max_tp + 255) / 256, B), 256, 0, st, d);
+        MVDR_LAUNCH_IF_CHAINED(chain, feat_compact_kernel, grid2(1, B), 1024, 0, st, d);
     }
-    MVDR_LAUNCH(term_offsets_kernel, grid2(1, B), 32, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, term_offsets_kernel, grid2(1, B), 32, 0, st, d);
     // node -> term
-    MVDR_LAUNCH(n2t_count_kernel, grid2(spread, B), 256, 0, st, d);
-    MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanN2T);
-    MVDR_LAUNCH(n2t_scatter_kernel, grid2(spread, B), 256, 0, st, d);
-    MVDR_LAUNCH(n2t_warp_sort_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
-    MVDR_LAUNCH(n2t_merge_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count * 12), B), 32 * kMergeWarps, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, n2t_count_kernel, grid2(spread, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanN2T);
+    MVDR_LAUNCH_IF_CHAINED(chain, n2t_scatter_kernel, grid2(spread, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, n2t_warp_sort_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, n2t_merge_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count * 12), B), 32 * kMergeWarps, 0, st, d);
     if (lc.cap_seg > kMergeMax)
-        MVDR_LAUNCH(n2t_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count), B), 256, (size_t)lc.cap_seg * 4, st, d);
+        MVDR_LAUNCH_IF_CHAINED(chain, n2t_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count), B), 256, (size_t)lc.cap_seg * 4, st, d);
     // node pair -> term
-    MVDR_LAUNCH(np_row_count_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
-    MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanRows);
-    MVDR_LAUNCH(np_row_build_kernel, grid2((lc.max_nodes + kRowWarps - 1) / kRowWarps, B), 32 * kRowWarps, 0, st, d);
-    MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanUpper);
-    MVDR_LAUNCH(np_half_compact_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
-    MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanBlkRows);
-    MVDR_LAUNCH(np_sym_scatter_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
-    MVDR_LAUNCH(np_lower_sort_kernel, grid2((lc.max_nodes + 3) / 4, B), 128, 0, st, d);
-    MVDR_LAUNCH(pair_order_kernel, grid2(min((lc.cap_pairs + kPairWindow - 1) / kPairWindow, spread), B), kLenBuckets, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, np_row_count_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanRows);
+    MVDR_LAUNCH_IF_CHAINED(chain, np_row_build_kernel, grid2((lc.max_nodes + kRowWarps - 1) / kRowWarps, B), 32 * kRowWarps, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanUpper);
+    MVDR_LAUNCH_IF_CHAINED(chain, np_half_compact_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanBlkRows);
+    MVDR_LAUNCH_IF_CHAINED(chain, np_sym_scatter_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, np_lower_sort_kernel, grid2((lc.max_nodes + 3) / 4, B), 128, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, pair_order_kernel, grid2(min((lc.cap_pairs + kPairWindow - 1) / kPairWindow, spread), B), kLenBuckets, 0, st, d);
     // bin-block CSR structure
-    MVDR_LAUNCH(bin_length_kernel, grid2((6 * lc.max_nodes / 32 + 256) / 256, B), 256, 0, st, d);
-    MVDR_LAUNCH(node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanBins);
-    MVDR_LAUNCH(bin_rowptr_kernel, grid2(spread, B), 256, 0, st, d);
-    MVDR_LAUNCH(bin_colptr_kernel, grid2((6 * lc.max_nodes + 255) / 256, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, bin_length_kernel, grid2((6 * lc.max_nodes / 32 + 256) / 256, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanBins);
+    MVDR_LAUNCH_IF_CHAINED(chain, bin_rowptr_kernel, grid2(spread, B), 256, 0, st, d);
+    MVDR_LAUNCH_IF_CHAINED(chain, bin_colptr_kernel, grid2((6 * lc.max_nodes + 255) / 256, B), 256, 0, st, d);
     return cudaGetLastError();
 }
 

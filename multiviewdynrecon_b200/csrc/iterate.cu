@@ -210,6 +210,7 @@ __device__ inline void fg_record(const InstDesc& I, uint32_t k, float4& o0, floa
 
 template <class T>
 __global__ void __launch_bounds__(256, 4) eval_terms_kernel(const InstDesc* insts, mvdr_penalty lam) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     TermOffsets off;
     off.load(I.counts);
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(256, 4) eval_terms_kernel(const InstDesc* inst
 // weighted squared residuals go to reduction region kRegDensityEnergy.
 template <class T>
 __global__ void __launch_bounds__(256, 2) eval_density_kernel(const InstDesc* insts, mvdr_penalty lam) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     const uint32_t Td = bad_inputs(I) ? 0u : I.counts->term_offset[0];
     double energy = 0;
@@ -2782,6 +2784,7 @@ __global__ void __launch_bounds__(192) bsr_apply_kernel(const InstDesc* insts, c
 // applyWarpFieldUpdateKernel (SolverIterationData.cu:9-57)
 template <bool MIXED>
 __global__ void __launch_bounds__(128) update_kernel(const InstDesc* insts) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < I.N; node += gridDim.x * blockDim.x) {
         float tw[6];
@@ -2859,6 +2862,7 @@ __global__ void __launch_bounds__(128) update_kernel(const InstDesc* insts) {
 // per-CTA partials summed in a fixed order (one CTA per instance)
 __global__ void __launch_bounds__(256) energy_sum_kernel(const InstDesc* insts, uint32_t count, uint32_t slot,
                                                          uint32_t density_count) {
+    chain_wait();
     const InstDesc& I = insts[blockIdx.y];
     __shared__ double ws[8];
     double e = 0;
@@ -2920,12 +2924,13 @@ static uint32_t eval_density_grid(const LaunchCfg& lc) {
 
 cudaError_t launch_eval_terms(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
     const uint32_t g = eval_terms_grid(lc);
-    if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH(eval_terms_kernel<double>, grid2(g, lc.B), 256, 0, st, d, lam);
-    else MVDR_LAUNCH(eval_terms_kernel<float>, grid2(g, lc.B), 256, 0, st, d, lam);
+    const bool chain = chain_kernels(lc);
+    if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH_IF_CHAINED(chain, eval_terms_kernel<double>, grid2(g, lc.B), 256, 0, st, d, lam);
+    else MVDR_LAUNCH_IF_CHAINED(chain, eval_terms_kernel<float>, grid2(g, lc.B), 256, 0, st, d, lam);
     if (lc.use_density) {
         const uint32_t gd = eval_density_grid(lc);
-        if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH(eval_density_kernel<double>, grid2(gd, lc.B), 256, 0, st, d, lam);
-        else MVDR_LAUNCH(eval_density_kernel<float>, grid2(gd, lc.B), 256, 0, st, d, lam);
+        if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH_IF_CHAINED(chain, eval_density_kernel<double>, grid2(gd, lc.B), 256, 0, st, d, lam);
+        else MVDR_LAUNCH_IF_CHAINED(chain, eval_density_kernel<float>, grid2(gd, lc.B), 256, 0, st, d, lam);
     }
     return cudaGetLastError();
 }
@@ -2935,18 +2940,11 @@ static uint32_t scale_grid(const LaunchCfg& lc) {
     return min((lc.cap_pairs + kScalePairsPerCta - 1) / kScalePairsPerCta, (uint32_t)lc.sm_count * 16);
 }
 
-// The kernels of a PCG iteration are launched chained for up to three instances, where
-// each takes 3 to 25 us and the gaps between them count: a 1,000-node frame in FP32 1281
-// -> 1117 us, a matrix-free one of 4,096 nodes 3784 -> 3370 us, 32,768 nodes 14.30 ->
-// 13.68 ms. In batches the waiting blocks hold places that the other lane's kernels
-// could use: 64 frames 10.17 -> 10.26 ms, an uneven batch 7.43 -> 7.63 ms.
-static bool chain_pcg(const LaunchCfg& lc) { return lc.B < 4; }
-
 // J.d then Jt.(J.d) (+ damping): `fused` takes the PCG direction of `parity`
 // as the operand and stores q with its d.q partials, else x -> y
 static void launch_apply_pair(const LaunchCfg& lc, InstDesc* d, const float* x, float* y, int parity, int fused,
                               uint32_t gterm, uint32_t gwarp, uint32_t B, const mvdr_penalty& lam, cudaStream_t st) {
-    const bool chain = fused && chain_pcg(lc);
+    const bool chain = fused && chain_kernels(lc);
     const bool mixed = lc.precision == MVDR_PRECISION_MIXED;
     if (mixed && lc.recompute_jr) {
         MVDR_LAUNCH_IF_CHAINED(chain, (apply_j_kernel<true, true>), grid2(gterm, B), 256, 0, st, d, x, parity, fused, lam);
@@ -3042,7 +3040,7 @@ cudaError_t launch_assemble_forked(const LaunchCfg& lc, InstDesc* d, const mvdr_
 }
 
 cudaError_t launch_energy(const LaunchCfg& lc, InstDesc* d, uint32_t slot, cudaStream_t st) {
-    MVDR_LAUNCH(energy_sum_kernel, grid2(1, lc.B), 256, 0, st, d, eval_terms_grid(lc), slot,
+    MVDR_LAUNCH_IF_CHAINED(chain_kernels(lc), energy_sum_kernel, grid2(1, lc.B), 256, 0, st, d, eval_terms_grid(lc), slot,
                 lc.use_density ? eval_density_grid(lc) : 0u);
     return cudaGetLastError();
 }
@@ -3150,7 +3148,7 @@ cudaError_t launch_pcg(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam
     if (scaled) MVDR_LAUNCH((pcg_init_kernel<true, true>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d);
     else if (mixed) MVDR_LAUNCH((pcg_init_kernel<true, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d);
     else MVDR_LAUNCH((pcg_init_kernel<false, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d);
-    const bool chain = chain_pcg(lc);
+    const bool chain = chain_kernels(lc);
     for (uint32_t it = 0; it < iters; ++it) {
         const int parity = (int)(it & 1u), first = it == 0;
         uint32_t nq;  // CTAs that store the d.q partials
@@ -3185,13 +3183,13 @@ cudaError_t launch_pcg(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam
 template <bool MIXED, uint32_t R, uint32_t S>
 static void spmv_shape_launch(const LaunchCfg& lc, InstDesc* d, int parity, cudaStream_t st) {
     auto* kernel = &pcg_spmv_kernel<MIXED, R, S>;
-    MVDR_LAUNCH_IF_CHAINED(chain_pcg(lc), kernel, grid2((lc.max_nodes + R - 1) / R, lc.B), 6 * S * R, 0, st, d, parity);
+    MVDR_LAUNCH_IF_CHAINED(chain_kernels(lc), kernel, grid2((lc.max_nodes + R - 1) / R, lc.B), 6 * S * R, 0, st, d, parity);
 }
 
 template <bool MIXED, uint32_t R, uint32_t S>
 static void spmv_col_launch(const LaunchCfg& lc, InstDesc* d, int parity, cudaStream_t st) {
     auto* kernel = &pcg_spmv_col_kernel<MIXED, R, S>;
-    MVDR_LAUNCH_IF_CHAINED(chain_pcg(lc), kernel, grid2((lc.max_nodes + R - 1) / R, lc.B), 6 * S * R, 0, st, d, parity);
+    MVDR_LAUNCH_IF_CHAINED(chain_kernels(lc), kernel, grid2((lc.max_nodes + R - 1) / R, lc.B), 6 * S * R, 0, st, d, parity);
 }
 
 template <bool MIXED>
@@ -3215,7 +3213,7 @@ static void spmv_dispatch(const LaunchCfg& lc, InstDesc* d, int parity, cudaStre
 template <uint32_t R, uint32_t S, uint32_t F>
 static void spmv_scaled_launch(const LaunchCfg& lc, InstDesc* d, int parity, cudaStream_t st) {
     auto* kernel = &pcg_spmv_scaled_kernel<R, S, F>;
-    MVDR_LAUNCH_IF_CHAINED(chain_pcg(lc), kernel, grid2((lc.max_nodes + R - 1) / R, lc.B), 6 * S * R, 0, st, d, parity);
+    MVDR_LAUNCH_IF_CHAINED(chain_kernels(lc), kernel, grid2((lc.max_nodes + R - 1) / R, lc.B), 6 * S * R, 0, st, d, parity);
 }
 
 // the shapes of kSpmvShapes for the scaled operator
@@ -3287,8 +3285,8 @@ cudaError_t launch_stage(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& l
 
 cudaError_t launch_update(const LaunchCfg& lc, InstDesc* d, cudaStream_t st) {
     const uint32_t g = (lc.max_nodes + 127) / 128;
-    if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH(update_kernel<true>, grid2(g, lc.B), 128, 0, st, d);
-    else MVDR_LAUNCH(update_kernel<false>, grid2(g, lc.B), 128, 0, st, d);
+    if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH_IF_CHAINED(chain_kernels(lc), update_kernel<true>, grid2(g, lc.B), 128, 0, st, d);
+    else MVDR_LAUNCH_IF_CHAINED(chain_kernels(lc), update_kernel<false>, grid2(g, lc.B), 128, 0, st, d);
     return cudaGetLastError();
 }
 
