@@ -733,46 +733,63 @@ __device__ inline uint32_t upper_entries_of(const InstDesc& I, const TermOffsets
     return c;
 }
 
-// warp per node: number of upper entries of the row, and n2t_w[p], the node's
+constexpr uint32_t kRowWarps = 4;  // of a CTA of the two row kernels
+
+// W warps (1, or the CTA's) per node: number of upper entries of the row, and n2t_w[p], the node's
 // skinning weight in each of its terms (0 for smooth; the values are those of
 // weight_of, PreconditionerBlocked.cu:23-29). The weights are inputs, recorded
 // once per solve, so that the assembly kernels read one coalesced value per entry
 // instead of the term's node and weight records.
-__global__ void __launch_bounds__(256) np_row_count_kernel(const InstDesc* insts) {
+template <uint32_t W>
+__global__ void __launch_bounds__(32 * kRowWarps) np_row_count_kernel(const InstDesc* insts) {
     chain_wait();
+    __shared__ uint32_t s_sum[kRowWarps];
     const InstDesc& I = insts[blockIdx.y];
     if (I.counts->node2term_entries > I.cap_k1) return;
     TermOffsets off;
     off.load(I.counts);
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); node < I.N; node += warps) {
-        const uint32_t b = I.n2t_offset[node], e = I.n2t_offset[node + 1];
+    constexpr uint32_t kNodes = kRowWarps / W;
+    const uint32_t warp = threadIdx.x >> 5, sub = warp % W;
+    for (uint32_t n0 = blockIdx.x * kNodes; n0 < I.N; n0 += gridDim.x * kNodes) {
+        const uint32_t node = n0 + warp / W;
         uint32_t c = 0;
+        if (node < I.N) {
+            const uint32_t b = I.n2t_offset[node], e = I.n2t_offset[node + 1];
 #pragma unroll 4
-        for (uint32_t p = b + lane_id(); p < e; p += 32) {
-            uint32_t k;
-            const TermType ty = off.typed(I.n2t_index[p], k);
-            const ushort4 n = term_nodes(I, ty, k);
-            float w = 0.f;
-            if (ty == kSmooth) {
-                // one pair (min, max), in the row of min; a node listed twice in
-                // the same smooth term gives no pair
-                const uint32_t o = n.x == node ? n.y : n.x;
-                c += o > node && o < I.N ? 1u : 0u;
-            } else {
-                if (ty != kInvalidTerm) w = weight_of(n, term_weights(I, ty, k), node);
-                const uint32_t a[4] = {n.x, n.y, n.z, n.w};
+            for (uint32_t p = b + 32 * sub + lane_id(); p < e; p += 32 * W) {
+                uint32_t k;
+                const TermType ty = off.typed(I.n2t_index[p], k);
+                const ushort4 n = term_nodes(I, ty, k);
+                float w = 0.f;
+                if (ty == kSmooth) {
+                    // one pair (min, max), in the row of min; a node listed twice in
+                    // the same smooth term gives no pair
+                    const uint32_t o = n.x == node ? n.y : n.x;
+                    c += o > node && o < I.N ? 1u : 0u;
+                } else {
+                    if (ty != kInvalidTerm) w = weight_of(n, term_weights(I, ty, k), node);
+                    const uint32_t a[4] = {n.x, n.y, n.z, n.w};
 #pragma unroll
-                for (int q = 0; q < 4; ++q) c += a[q] > node && a[q] < I.N ? 1u : 0u;
+                    for (int q = 0; q < 4; ++q) c += a[q] > node && a[q] < I.N ? 1u : 0u;
+                }
+                I.n2t_w[p] = w;
             }
-            I.n2t_w[p] = w;
+            c = warp_sum(c);
+            if (W == 1 && lane_id() == 0) I.row_count[node] = c;
         }
-        c = warp_sum(c);
-        if (lane_id() == 0) I.row_count[node] = c;
+        if constexpr (W > 1) {
+            if (lane_id() == 0) s_sum[warp] = c;
+            __syncthreads();
+            if (sub == 0 && lane_id() == 0 && node < I.N) {
+                for (uint32_t w = 1; w < W; ++w) c += s_sum[warp + w];
+                I.row_count[node] = c;
+            }
+            __syncthreads();
+        }
     }
 }
 
-// Warp per node: the row's (j, t) entries, j > node, in ascending (j, t) order
+// W warps per node: the row's (j, t) entries, j > node, in ascending (j, t) order
 // without sorting, with the products of the two nodes' weights. The node's term
 // list is already ascending in t. A first pass counts the entries of each
 // distinct partner in a small hash table in shared memory; the partners are
@@ -784,27 +801,31 @@ __global__ void __launch_bounds__(256) np_row_count_kernel(const InstDesc* insts
 // nodes the same 101, with one 580 and 118. A term that lists a partner twice, or a
 // node with more than kRowPartners partners, takes the sweep (one pass over the
 // list per partner), which is what every node took before: 285 -> 101 us on a
-// 500-node frame, whose lists reach 1,276 terms, 72 -> 51 us on 3,000 nodes, 752 ->
-// 606 us on 32,768, with the weights' own pass (77, 42 and 219 us) saved. Writes
-// np_index, np_scale, the per-pair (key, start) of the row and upper_count.
-constexpr uint32_t kRowSlices = 2, kRowTable = 256, kRowPartners = 192, kRowWarps = 4;
+// 500-node frame, whose lists reach 1,276 terms (54 with a CTA per node), 72 -> 51 us
+// on 4,096 nodes, 752 -> 606 us on 32,768, with the weights' own pass (77, 42 and 219
+// us) saved. Writes np_index, np_scale, the per-pair (key, start) of the row and
+// upper_count.
+constexpr uint32_t kRowSlices = 2, kRowPartners = 192;
 
-struct RowTable {
-    uint32_t key[kRowTable];    // partner, kInvalid: free
-    uint32_t count[kRowTable];  // its entries, then the place of its next one
-    uint32_t mask[kRowTable];   // lanes of the current slice that hold it
+// W warps of a CTA share the table and a node's list, a run of it each
+template <uint32_t W> struct RowTable {
+    static constexpr uint32_t kBits = W == 1 ? 8 : 9, kSize = 1u << kBits;
+    // every thread may pass the test of `used` before the others' insertions count
+    static_assert(kRowPartners + 32 * W < kSize, "a free entry must remain");
+    uint32_t key[kSize];       // partner, kInvalid: free
+    uint32_t count[W][kSize];  // its entries in the warp's run, then the place of the next one
+    uint32_t mask[W][kSize];   // lanes of the warp's current slice that hold it
     uint32_t slot[kRowPartners], rank_slot[kRowPartners];  // the used slots, then in order of the partner
     uint32_t used, sweep;
+
+    __device__ static uint32_t hash(uint32_t j) { return (j * 2654435761u) >> (32 - kBits); }
+    __device__ static uint32_t next(uint32_t h) { return (h + 1) & (kSize - 1); }
+    __device__ uint32_t find(uint32_t j) const {
+        uint32_t h = hash(j);
+        while (key[h] != j) h = next(h);
+        return h;
+    }
 };
-
-__device__ inline uint32_t row_hash(uint32_t j) { return (j * 2654435761u) >> 24; }
-static_assert(kRowTable == 256, "eight hash bits");
-
-__device__ inline uint32_t row_find(const RowTable& tb, uint32_t j) {
-    uint32_t h = row_hash(j);
-    while (tb.key[h] != j) h = (h + 1) & (kRowTable - 1);
-    return h;
-}
 
 // weight product of an entry's two nodes, exact in double (0 for a smooth term)
 __device__ inline double pair_scale(const InstDesc& I, const TermOffsets& off, uint32_t t, uint32_t i, uint32_t j) {
@@ -853,34 +874,47 @@ __device__ inline uint32_t row_sweep(const InstDesc& I, const TermOffsets& off, 
     }
 }
 
+template <uint32_t W>
 __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const InstDesc* insts) {
     chain_wait();
-    __shared__ RowTable s_table[kRowWarps];
+    static_assert(W == 1 || W == kRowWarps, "a warp or the CTA");
+    using Table = RowTable<W>;
+    __shared__ Table s_table[kRowWarps / W];
     const InstDesc& I = insts[blockIdx.y];
     const DeviceCounts* C = I.counts;
     if (C->node2term_entries > I.cap_k1 || C->nodepair_entries > I.cap_k2) return;
     TermOffsets off;
     off.load(I.counts);
     const uint32_t lane = lane_id(), lt_mask = (1u << lane) - 1u;
-    RowTable& tb = s_table[threadIdx.x >> 5];
-    const uint32_t warps = gridDim.x * kRowWarps;
-    for (uint32_t node = blockIdx.x * kRowWarps + (threadIdx.x >> 5); node < I.N; node += warps) {
+    const uint32_t warp = threadIdx.x >> 5, sub = warp % W, member = 32 * sub + lane;
+    Table& tb = s_table[warp / W];
+    uint32_t* const count = tb.count[sub];
+    uint32_t* const mask = tb.mask[sub];
+    auto sync = [] {
+        if constexpr (W == 1) __syncwarp();
+        else __syncthreads();
+    };
+    constexpr uint32_t kNodes = kRowWarps / W;  // (W > 1: the same node for every thread)
+    for (uint32_t node = blockIdx.x * kNodes + warp / W; node < I.N; node += gridDim.x * kNodes) {
         const uint32_t b0 = I.n2t_offset[node], b1 = I.n2t_offset[node + 1];
         const uint32_t out = I.row_offset[node], len = I.row_count[node];
-        for (uint32_t i = lane; i < kRowTable; i += 32) {
+        // this warp's run of the list
+        const uint32_t run = (b1 - b0 + 32 * W - 1) / (32 * W) * 32;
+        const uint32_t c0 = min(b0 + sub * run, b1), c1 = min(c0 + run, b1);
+        for (uint32_t i = member; i < Table::kSize; i += 32 * W) {
             tb.key[i] = kInvalid;
-            tb.count[i] = 0;
-            tb.mask[i] = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < W; ++w) tb.count[w][i] = tb.mask[w][i] = 0;
         }
-        if (lane == 0) tb.used = tb.sweep = 0;
-        __syncwarp();
+        if (member == 0) tb.used = tb.sweep = 0;
+        sync();
         // the partners above `node` of the terms of kRowSlices slices
         uint32_t t[kRowSlices], js[kRowSlices][4];
         auto load = [&](uint32_t base) {
 #pragma unroll
             for (uint32_t s = 0; s < kRowSlices; ++s) {
                 const uint32_t p = base + 32 * s + lane;
-                t[s] = p < b1 ? I.n2t_index[p] : kInvalid;
+                t[s] = p < c1 ? I.n2t_index[p] : kInvalid;
             }
 #pragma unroll
             for (uint32_t s = 0; s < kRowSlices; ++s) {
@@ -899,7 +933,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const I
             }
         };
         bool sweep = false;
-        for (uint32_t base = b0; base < b1 && !sweep; base += 32 * kRowSlices) {
+        for (uint32_t base = c0; base < c1 && !sweep; base += 32 * kRowSlices) {
             load(base);
 #pragma unroll
             for (uint32_t s = 0; s < kRowSlices; ++s) {
@@ -914,7 +948,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const I
                         tb.sweep = 1;
                         continue;
                     }
-                    uint32_t h = row_hash(j);
+                    uint32_t h = Table::hash(j);
                     for (;;) {
                         const uint32_t seen = atomicCAS(&tb.key[h], kInvalid, j);
                         if (seen == j) break;
@@ -923,46 +957,56 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const I
                             if (u < kRowPartners) tb.slot[u] = h;
                             break;
                         }
-                        h = (h + 1) & (kRowTable - 1);
+                        h = Table::next(h);
                     }
-                    atomicAdd(&tb.count[h], 1u);
+                    atomicAdd(&count[h], 1u);
                 }
             }
             __syncwarp();
-            sweep = __any_sync(0xffffffffu, tb.sweep != 0);  // (the same in every lane)
+            sweep = __any_sync(0xffffffffu, *(volatile uint32_t*)&tb.sweep != 0);  // (the same in every lane)
         }
-        __syncwarp();
+        sync();
         const uint32_t used = tb.used;
-        if (sweep || used > kRowPartners) {
-            const uint32_t runs = row_sweep(I, off, node, b0, b1, out, len);
-            if (lane == 0) I.upper_count[node] = runs;
-            __syncwarp();
+        if (tb.sweep || used > kRowPartners) {
+            if (sub == 0) {
+                const uint32_t runs = row_sweep(I, off, node, b0, b1, out, len);
+                if (lane == 0) I.upper_count[node] = runs;
+            }
+            sync();
             continue;
         }
-        // rank the partners; starts in that order
-        for (uint32_t i = lane; i < used; i += 32) {
+        // rank the partners; starts in that order, within a partner in order of the runs
+        for (uint32_t i = member; i < used; i += 32 * W) {
             const uint32_t h = tb.slot[i], j = tb.key[h];
             uint32_t rank = 0;
             for (uint32_t m = 0; m < used; ++m) rank += tb.key[tb.slot[m]] < j ? 1u : 0u;
             tb.rank_slot[rank] = h;
         }
-        __syncwarp();
-        uint32_t start = 0;
-        for (uint32_t base = 0; base < used; base += 32) {
-            const uint32_t r = base + lane;
-            const uint32_t h = r < used ? tb.rank_slot[r] : 0u, n = r < used ? tb.count[h] : 0u;
-            const uint32_t incl = warp_inclusive_scan(n);
-            if (r < used) {
-                I.tmp_key[out + r] = node * I.enc + tb.key[h];
-                I.tmp_start[out + r] = out + start + incl - n;
-                tb.count[h] = start + incl - n;
+        sync();
+        if (sub == 0) {
+            uint32_t start = 0;
+            for (uint32_t base = 0; base < used; base += 32) {
+                const uint32_t r = base + lane, h = r < used ? tb.rank_slot[r] : 0u;
+                uint32_t n = 0;
+                for (uint32_t w = 0; w < W; ++w) n += r < used ? tb.count[w][h] : 0u;
+                const uint32_t incl = warp_inclusive_scan(n);
+                uint32_t place = start + incl - n;
+                if (r < used) {
+                    I.tmp_key[out + r] = node * I.enc + tb.key[h];
+                    I.tmp_start[out + r] = out + place;
+                    for (uint32_t w = 0; w < W; ++w) {
+                        const uint32_t own = tb.count[w][h];
+                        tb.count[w][h] = place;
+                        place += own;
+                    }
+                }
+                start += __shfl_sync(0xffffffffu, incl, 31);
             }
-            start += __shfl_sync(0xffffffffu, incl, 31);
+            if (lane == 0) I.upper_count[node] = used;
         }
-        if (lane == 0) I.upper_count[node] = used;
-        __syncwarp();
+        sync();
         // place the entries
-        for (uint32_t base = b0; base < b1; base += 32 * kRowSlices) {
+        for (uint32_t base = c0; base < c1; base += 32 * kRowSlices) {
             load(base);
             float4 w4[kRowSlices];
             ushort4 kn[kRowSlices];
@@ -981,8 +1025,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const I
                 for (int q = 0; q < 4; ++q) {
                     h[q] = kInvalid;
                     if (js[s][q] == kInvalid) continue;
-                    h[q] = row_find(tb, js[s][q]);
-                    atomicOr(&tb.mask[h[q]], 1u << lane);
+                    h[q] = tb.find(js[s][q]);
+                    atomicOr(&mask[h[q]], 1u << lane);
                 }
                 __syncwarp();
                 const double wi = (double)weight_of(kn[s], w4[s], node);
@@ -990,8 +1034,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const I
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     if (h[q] == kInvalid) continue;
-                    m[q] = tb.mask[h[q]];
-                    const uint32_t at = tb.count[h[q]] + __popc(m[q] & lt_mask);
+                    m[q] = mask[h[q]];
+                    const uint32_t at = count[h[q]] + __popc(m[q] & lt_mask);
                     if (at < len) {
                         I.np_index[out + at] = t[s];
                         I.np_scale[out + at] = wi * (double)weight_of(kn[s], w4[s], js[s][q]);
@@ -1001,13 +1045,13 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) np_row_build_kernel(const I
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {  // the partner's first lane moves its place on
                     if (h[q] == kInvalid || (m[q] & lt_mask)) continue;
-                    tb.count[h[q]] += __popc(m[q]);
-                    tb.mask[h[q]] = 0;
+                    count[h[q]] += __popc(m[q]);
+                    mask[h[q]] = 0;
                 }
                 __syncwarp();
             }
         }
-        __syncwarp();
+        sync();
     }
 }
 
@@ -1230,6 +1274,12 @@ cudaError_t set_index_smem_limits(size_t seg_bytes) {
     return cudaFuncSetAttribute(n2t_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_bytes);
 }
 
+// A CTA per node in the row kernels, while there are few nodes, whose lists are long.
+// Whole solves, us, with a warp / a CTA per node: 500 nodes 801 / 714, 800 2600 / 2417,
+// 1,500 1845 / 1775, 2,200 1675 / 1600, 3,001 1571 / 1547, 4,096 1495 / 1500; 32,768 13705 /
+// 13800, 16 x 4,096 10140 / 10470.
+static bool wide_rows(const LaunchCfg& lc) { return (uint64_t)lc.B * lc.max_nodes < 4096; }
+
 cudaError_t launch_build_index(const LaunchCfg& lc, InstDesc* d, cudaStream_t st) {
     const uint32_t B = lc.B;
     const uint32_t cpv = lc.chunks_per_view;
@@ -1259,9 +1309,13 @@ cudaError_t launch_build_index(const LaunchCfg& lc, InstDesc* d, cudaStream_t st
     if (lc.cap_seg > kMergeMax)
         MVDR_LAUNCH_IF_CHAINED(chain, n2t_sort_kernel, grid2(min(lc.max_nodes, (uint32_t)lc.sm_count), B), 256, (size_t)lc.cap_seg * 4, st, d);
     // node pair -> term
-    MVDR_LAUNCH_IF_CHAINED(chain, np_row_count_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
+    const bool wide = wide_rows(lc);
+    const dim3 grow = grid2(wide ? lc.max_nodes : (lc.max_nodes + kRowWarps - 1) / kRowWarps, B);
+    if (wide) MVDR_LAUNCH_IF_CHAINED(chain, np_row_count_kernel<kRowWarps>, grow, 32 * kRowWarps, 0, st, d);
+    else MVDR_LAUNCH_IF_CHAINED(chain, np_row_count_kernel<1>, grow, 32 * kRowWarps, 0, st, d);
     MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanRows);
-    MVDR_LAUNCH_IF_CHAINED(chain, np_row_build_kernel, grid2((lc.max_nodes + kRowWarps - 1) / kRowWarps, B), 32 * kRowWarps, 0, st, d);
+    if (wide) MVDR_LAUNCH_IF_CHAINED(chain, np_row_build_kernel<kRowWarps>, grow, 32 * kRowWarps, 0, st, d);
+    else MVDR_LAUNCH_IF_CHAINED(chain, np_row_build_kernel<1>, grow, 32 * kRowWarps, 0, st, d);
     MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanUpper);
     MVDR_LAUNCH_IF_CHAINED(chain, np_half_compact_kernel, grid2((lc.max_nodes + 7) / 8, B), 256, 0, st, d);
     MVDR_LAUNCH_IF_CHAINED(chain, node_scan_kernel, grid2(1, B), 1024, 0, st, d, (int)kScanBlkRows);

@@ -38,9 +38,20 @@ def _crowded(nodes, twice):
     (lambda: _crowded(60, True), (None, None)),          # a node twice in a term
 ])
 def test_index_equals_the_oracle(scene, long_lists, oracle_mod):
+    _check(scene(), long_lists, oracle_mod, None)
+
+
+@pytest.mark.parametrize("max_nodes", [4095, 4096])  # a CTA or a warp per row
+@pytest.mark.parametrize("scene", [lambda: _few_nodes(40, 96, 72), lambda: _crowded(230, False),
+                                   lambda: _crowded(60, True)])
+def test_index_at_the_change_of_row_kernels(scene, max_nodes, oracle_mod):
+    _check(scene(), (None, None), oracle_mod, max_nodes)
+
+
+def _check(scene, long_lists, oracle_mod, max_nodes):
     from multiviewdynrecon_b200.solver import NonRigidSolver
-    scene = scene()
     cfg = abi.make_config(scene)
+    cfg.max_nodes = max_nodes or cfg.max_nodes
     cfg.max_node_pairs = max(16 * scene.num_nodes, scene.num_nodes ** 2)
     cfg.max_terms_per_node = 16384
     g = NonRigidSolver(cfg)
