@@ -1198,7 +1198,8 @@ __global__ void __launch_bounds__(kPairChunk, 7) offdiag_group_kernel(const Inst
     const uint32_t windows = pair_slots(I.counts->half_pairs) / kPairWindow, group = threadIdx.x >> 4;
     for (uint32_t item = blockIdx.x; item < windows * (share / kPairGroups); item += gridDim.x) {
         // (pairs of about equal length in a warp's two groups)
-        const uint32_t pos = (item % windows) * kPairChunk + (item / windows) * kPairGroups + group;
+        const uint32_t rank = item / windows * kPairGroups + group;  // in the window
+        const uint32_t pos = (rank / kPairChunk * windows + item % windows) * kPairChunk + rank % kPairChunk;
         pair_by_group<Acc, DENS>(I, off, lam, I.pair_order[pos], s_stage[0][group], s_stage[DENS ? 1 : 0][group],
                                  BlockStore<MIXED>::ptr(I));
     }
@@ -1213,7 +1214,7 @@ __global__ void __launch_bounds__(kPairChunk, 4) offdiag_thread_kernel(const Ins
     off.load(I.counts);
     const uint32_t slots = pair_slots(I.counts->half_pairs), first = slots / kPairWindow * kPairChunk;
     for (uint32_t pos = blockIdx.x * kPairChunk + threadIdx.x; pos < slots; pos += gridDim.x * kPairChunk) {
-        if (pos < first && threadIdx.x < share) continue;
+        if (pos / first * kPairChunk + threadIdx.x < share) continue;  // (its rank in the window)
         const uint32_t h = I.pair_order[pos];
         if (h != kInvalid) pair_by_thread<typename BlockStore<MIXED>::V>(I, off, lam, h, BlockStore<MIXED>::ptr(I));
     }
@@ -2975,13 +2976,17 @@ static void launch_diag(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& la
 }
 
 // Pairs of each window taken by group. By group a pair's chain is five times
-// shorter but its entries cost seven times the instructions: an eighth of the
-// pairs while the launch is bound by its chains; few where it has other work to
-// fill the GPU meanwhile. Whole solves, ms, with 128 / 32 / 8 of 1024: 500-node
-// frame 1.49 / 1.63 / -, 4096-node frame 2.38 / 2.52 / -, 32,768-node frame 16.2 /
-// 15.8 / -, 16 x 4096 nodes in two lanes 10.74 / 10.53 / 10.31.
+// shorter but its entries cost seven times the instructions: half of the pairs
+// while the launch is bound by its chains (few nodes, long lists); few where it has
+// other work to fill the GPU meanwhile. Whole solves, us, with 512 / 256 / 128 / 32
+// of 1024: 500 nodes 1967 / 2470 / 3054 / -, 1,000 1558 / 1783 / 2080 / -, 4,096 1407 /
+// 1439 / 1518 / -, 6,000 1957 / 1924 / 1977 / 2080, 9,000 2279 / 2217 / 2188 / 2184, 13,000
+// 2421 / 2347 / 2312 / 2280; larger images, ms, 8,000 11.1 / 11.3 / 13.8 / 16.4, 16,000 12.3
+// / 12.15 / 12.0 / 12.1, 32,768 (128 / 32) 16.2 / 15.8; 16 x 4,096 nodes in two lanes (128 /
+// 32 / 8) 10.74 / 10.53 / 10.31.
 static uint32_t group_share(const LaunchCfg& lc) {
-    if ((uint64_t)lc.B * lc.max_nodes < 16384) return kPairChunk;
+    const uint64_t nodes = (uint64_t)lc.B * lc.max_nodes;
+    if (nodes < 16384) return nodes < 5120 ? 512 : nodes < 10240 ? 256 : 128;
     return lc.B < 4 ? 32 : 8;
 }
 // the off-diagonal blocks: the long pairs (by group), the others (by thread)

@@ -75,3 +75,24 @@ def test_upper_blocks_at_every_pair_length(precision, nodes, width, height):
     half_ulps = length + 8 if precision == abi.PRECISION_FP32 else np.full(len(length), 2)
     assert np.all(np.abs(got - want) <= half_ulps[:, None, None] * 2.0 ** -24 * size + 1e-30)
     g.close()
+
+
+def test_blocks_do_not_depend_on_the_share_taken_by_group():
+    """max_nodes sets how many pairs of a window go to the 16-lane groups (512, 256,
+    128 or 32 of 1024); both forms give the same bits."""
+    from multiviewdynrecon_b200.solver import NonRigidSolver
+    scene = synth.torso_multi_view(seed=3, num_nodes=400, num_views=2, width=160, height=120, features_per_view=40,
+                                   cross_per_pair=40)
+    got = []
+    for max_nodes in (400, 5119, 5120, 10239, 10240, 16383, 16384):
+        cfg = abi.make_config(scene)
+        cfg.max_nodes = max_nodes
+        solver = NonRigidSolver(cfg)
+        solver.set_solver_input(scene)
+        solver.build_index()
+        solver.gn_iteration(5)
+        got.append(solver.get_array(abi.ARRAY_OFFDIAG_BLOCKS))
+        assert solver.counts().half_pairs > 1024  # several windows
+        solver.close()
+    for blocks in got[1:]:
+        assert np.array_equal(blocks, got[0])
