@@ -2620,7 +2620,11 @@ __global__ void __launch_bounds__(256, RECOMP ? 2 : 4) apply_j_kernel(const Inst
     const typename PcgVec<MIXED>::T* dv = PcgVec<MIXED>::d(I, parity);
     // mixed precision keeps J.p in double (jp holds 3 doubles per term)
     Acc* jp = reinterpret_cast<Acc*>(I.jp);
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < T; i += gridDim.x * blockDim.x) {
+        // The terms that are no pixels take longest (a chain of loads per node): they
+        // go first, not at the end of the last wave, which makes a 4,096-node
+        // matrix-free frame 3290 -> 3093 us.
+        const uint32_t t = i < T - off.o[0] ? i + off.o[0] : i - (T - off.o[0]);
         uint32_t k;
         const TermType ty = off.typed(t, k);
         const ushort4 nn = term_nodes(I, ty, k);
@@ -2667,7 +2671,9 @@ __global__ void __launch_bounds__(256, RECOMP ? 2 : 4) apply_j_kernel(const Inst
             const int ch = term_rows(I, off, lam, t, node, tr);
             Acc p[6];
             load_node6<Acc>(fused, dv, xin, node, p);
-            for (int c = 0; c < ch; ++c) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (c >= ch) break;
                 Acc a = 0;
 #pragma unroll
                 for (int i = 0; i < 6; ++i) a += (Acc)tr.J[c][i] * p[i];
@@ -2733,7 +2739,9 @@ __global__ void __launch_bounds__(256, RECOMP ? 2 : 4) apply_jt_kernel(const Ins
             TermRows tr;
             const int ch = term_rows(I, off, lam, t, node, tr);
             const T sc = (T)tr.lam2 * (T)tr.w;
-            for (int c = 0; c < ch; ++c) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (c >= ch) break;
                 const T y = jp[(size_t)c * Tn + t];
 #pragma unroll
                 for (int i = 0; i < 6; ++i) acc[i] += sc * (T)tr.J[c][i] * y;
