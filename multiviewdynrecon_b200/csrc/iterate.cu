@@ -1230,7 +1230,7 @@ __global__ void __launch_bounds__(kPairChunk, 4) offdiag_thread_kernel(const Ins
 // 1e-4 to 5e-4. In exact arithmetic the iterates are those of block-Jacobi PCG
 // on A (BlockPCG.cuh:65-181): x = L^-T x^, r^ = L^-1 r, and r^.r^ = r.M^-1 r.
 // This kernel forms A^_ij from the double block A_ij (i < j) that
-// offdiag_kernel stored: 8 lanes per pair, lane k of the first six solves
+// the off-diagonal kernels stored: 8 lanes per pair, lane k of the first six solves
 // column k of L_i Y = A_ij, the pair's lanes exchange Y through shared memory,
 // and lane k then solves L_j z = Y(k, :)^T, which is row k of A^_ij.
 constexpr uint32_t kScalePairsPerCta = 16;

@@ -34,9 +34,9 @@ inline void launch_chained(void (*kernel)(P...), dim3 grid, uint32_t block, size
 
 // The kernels of a solve are launched chained for up to three instances, where each
 // takes 2 to 25 us and the gaps between them count. us, plain / PCG chained / all: a
-// 500-node frame 842 / 842 / 801, 1,000 nodes in FP32 1281 / 1117 / 1063, 4,096 nodes 1566
+// 500-node frame 842 / 842 / 801, 2,048 nodes in FP32 1281 / 1117 / 1063, 4,096 nodes 1566
 // / 1566 / 1463 and matrix-free 3784 / 3370 / 3300, 32,768 nodes 14300 / 13680 / 13700. In
-// batches the waiting blocks hold places that the other lane's kernels could use: 64
+// batches the waiting blocks hold places that the other lane's kernels could use: 16
 // frames 10.17 -> 10.26 ms, an uneven batch 7.43 -> 7.63 ms. For the same reason the
 // factorisation, next to which other branches of the assembly run, is launched plainly
 // (chained: 1512 us for 4,096 nodes), as is a kernel that follows a join of streams.
