@@ -170,7 +170,7 @@ __device__ inline DQ dq_pow_scale(const DQ& d, float ratio) {
 // the row-major M34
 __device__ inline M34 load_mat34(const mvdr_mat34* p) {
     const float4* q = reinterpret_cast<const float4*>(p);
-    const float4 a = q[0], b = q[1], c = q[2];
+    const float4 a = __ldcs(q), b = __ldcs(q + 1), c = __ldcs(q + 2);
     const float f[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
     M34 m;
     for (int r = 0; r < 3; ++r)
@@ -242,25 +242,30 @@ __global__ void __launch_bounds__(256) forward_warp_kernel(const __grid_constant
     }
 }
 
+// Bound by memory (136 bytes a surfel): everything a thread reads of its own is loaded
+// before the field's gathers, and all of it streams past the caches that hold the
+// field. 4.0M surfels with corrections: 97 -> 86 us, 6.3 TB/s.
 __global__ void __launch_bounds__(256) inverse_warp_kernel(const __grid_constant__ WarpArgs a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.S) return;
-    const ushort4 knn = a.knn[i];
-    const float4 v = a.in_v[i], n = a.in_n[i];
+    const ushort4 knn = __ldcs(a.knn + i);
+    const float4 v = __ldcs(a.in_v + i), n = __ldcs(a.in_n + i), w = __ldcs(a.w + i);
+    M34 correct;
+    if (a.correct) correct = load_mat34(a.correct + i);
     float3 p = make_float3(kNaN, kNaN, kNaN), q = p;
     if (knn_ok(knn, a.num_field)) {
-        const M34 se3 = se3_of_normalized(normalized(blend(a.field, knn, a.w[i])));
+        const M34 se3 = se3_of_normalized(normalized(blend(a.field, knn, w)));
         // apply_inversed_se3: R^T (v - t)
         p = rotT3(se3, make_float3(v.x - se3.t[0], v.y - se3.t[1], v.z - se3.t[2]));
         q = rotT3(se3, xyz(n));
         if (a.correct) {
-            const M34 ci = inverse34(load_mat34(a.correct + i));
+            const M34 ci = inverse34(correct);
             p = apply3(ci, p);
             q = rot3(ci, q);
         }
     }
-    a.out_v[i] = make_float4(p.x, p.y, p.z, v.w);
-    a.out_n[i] = make_float4(q.x, q.y, q.z, n.w);
+    __stcs(a.out_v + i, make_float4(p.x, p.y, p.z, v.w));
+    __stcs(a.out_n + i, make_float4(q.x, q.y, q.z, n.w));
 }
 
 // ------------------------------------------------------------ node error ----
