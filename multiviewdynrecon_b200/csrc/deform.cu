@@ -373,10 +373,13 @@ __device__ inline unsigned long long to_fixed(float v) {
 // the 18 window loads, of which those of the normals now stop at the first match. So
 // the warp first adds up its pixels' contributions to each distinct node. The sums
 // are integers: exact, whatever the order. A value below 2^50 is added as two limbs
-// of 26 bits, of which 32 x 4 fit 32-bit sums; a warp with a larger or negative one
-// adds pixel by pixel. Five views of 1280 x 720, 32,768 nodes: 364 -> 282 us, now
-// bound by issuing its instructions.
+// of 25 bits, because a node may be all four of a surfel's (a scene of one node) and
+// so be added 32 x 4 times; a warp with a larger or negative value adds pixel by
+// pixel. Five views of 1280 x 720, 32,768 nodes: 364 -> 282 us, now bound by issuing
+// its instructions.
 constexpr uint32_t kTileX = 32, kTileY = 8;  // pixels of a CTA
+constexpr uint32_t kLimbBits = 25, kLimbMask = (1u << kLimbBits) - 1u;
+static_assert(32ull * 4 * kLimbMask <= 0xFFFFFFFFull, "a warp's sum of one limb fits 32 bits");
 
 __global__ void __launch_bounds__(256) node_error_kernel(const InstDesc* __restrict__ insts, uint32_t inst,
                                                          const __grid_constant__ NodeErrArgs a) {
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(256) node_error_kernel(const InstDesc* __restr
         }
         all |= es[k] | ws[k];
     }
-    if (__any_sync(0xffffffffu, (all >> 50) != 0)) {
+    if (__any_sync(0xffffffffu, (all >> (2 * kLimbBits)) != 0)) {
         if (err > 1e-6f) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -415,14 +418,13 @@ __global__ void __launch_bounds__(256) node_error_kernel(const InstDesc* __restr
         }
         return;
     }
-    constexpr uint32_t kLimb = (1u << 26) - 1u;
     uint32_t limb[4][4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        limb[k][0] = (uint32_t)es[k] & kLimb;
-        limb[k][1] = (uint32_t)(es[k] >> 26);
-        limb[k][2] = (uint32_t)ws[k] & kLimb;
-        limb[k][3] = (uint32_t)(ws[k] >> 26);
+        limb[k][0] = (uint32_t)es[k] & kLimbMask;
+        limb[k][1] = (uint32_t)(es[k] >> kLimbBits);
+        limb[k][2] = (uint32_t)ws[k] & kLimbMask;
+        limb[k][3] = (uint32_t)(ws[k] >> kLimbBits);
     }
     for (;;) {
         const uint32_t node = __reduce_min_sync(0xffffffffu, min(min(nk[0], nk[1]), min(nk[2], nk[3])));
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(256) node_error_kernel(const InstDesc* __restr
         for (int l = 0; l < 4; ++l) sum[l] = __reduce_add_sync(0xffffffffu, sum[l]);
         if (lane < 2) {
             const uint32_t low = lane ? sum[2] : sum[0], high = lane ? sum[3] : sum[1];
-            atomicAdd(a.acc + (lane ? N : 0u) + node, ((unsigned long long)high << 26) + low);
+            atomicAdd(a.acc + (lane ? N : 0u) + node, ((unsigned long long)high << kLimbBits) + low);
         }
     }
 }

@@ -34,3 +34,28 @@ def test_node_error_equals_the_oracle(oracle_mod, width, height, weights):
         assert np.array_equal(got[k][0].cpu().numpy(), want[k][0], equal_nan=True), k
     assert (want["accumulated_error"] != 0).sum() > 10
     solver.close()
+
+
+@pytest.mark.parametrize("width,height,nodes,times", [(97, 65, 1, 4), (96, 64, 2, 3), (129, 57, 40, 3), (65, 67, 40, 4)])
+def test_node_error_of_surfels_that_repeat_a_node(oracle_mod, width, height, nodes, times):
+    """A node three or four times among each surfel's four, as every scene of one or
+    two nodes has it: up to 128 entries of a tile for one node."""
+    scene = synth.sphere_single_view(seed=4, num_nodes=40, width=width, height=height)
+    rng = np.random.default_rng(8)
+    scene.canonical_nodes, scene.node_se3 = scene.canonical_nodes[:nodes], scene.node_se3[:nodes]
+    scene.node_graph = scene.node_graph[:0]
+    scene.surfel_knn_weight[:] = rng.uniform(0.05, 0.4, scene.surfel_knn_weight.shape)
+    scene.surfel_knn[:] %= nodes
+    for column in range(1, times):
+        scene.surfel_knn[:, column] = scene.surfel_knn[:, 0]
+    solver = NonRigidSolver(abi.make_config(scene))
+    solver.set_solver_input(scene)
+    got = solver.compute_alignment_error_on_nodes(maps=True)
+    torch.cuda.synchronize()
+    want = oracle_mod.node_error(scene, scene.node_se3, maps=True)
+    for k in ("accumulated_error", "accumulated_weight", "united_error", "large_error_mark"):
+        assert np.array_equal(got[k].cpu().numpy().astype(want[k].dtype), want[k], equal_nan=True), k
+    for k in ("alignment_error_map", "node_error_map"):
+        assert np.array_equal(got[k][0].cpu().numpy(), want[k][0], equal_nan=True), k
+    assert (want["accumulated_weight"] > 10).any()
+    solver.close()
