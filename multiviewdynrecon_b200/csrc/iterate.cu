@@ -3074,6 +3074,16 @@ static uint32_t spmv_grid(const LaunchCfg& lc) {
     return (lc.max_nodes + R - 1) / R;
 }
 
+uint32_t partial_slots(const LaunchCfg& lc) {
+    // the terms' and the matrix-free grids, and the persistent PCG's (256 threads a CTA)
+    uint32_t n = (uint32_t)lc.sm_count * 8;
+    // a warp per node in CTAs of eight (apply_jt_kernel); the resident PCG's tiles
+    n = max(n, (lc.max_nodes + 7) / 8);
+    n = max(n, (lc.max_nodes + kResidentRows - 1) / kResidentRows * (kResidentRows / kResidentTile));
+    for (const SpmvShape& shape : kSpmvShapes) n = max(n, (lc.max_nodes + shape.rows - 1) / shape.rows);
+    return n;
+}
+
 uint32_t persistent_pcg_grid(int mixed, int sm_count) {
     int nb = 0;
     const cudaError_t e =

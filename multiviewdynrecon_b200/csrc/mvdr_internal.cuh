@@ -395,6 +395,10 @@ void count_launch();
 // co-resident CTAs of the persistent PCG kernel on this device (0 on error)
 uint32_t persistent_pcg_grid(int mixed, int sm_count);
 
+// slots of a region of the per-CTA partial sums: as many as the largest launch of
+// this configuration stores, whichever SpMV shape is chosen
+uint32_t partial_slots(const LaunchCfg& lc);
+
 // whether this configuration's PCG can run as one launch with the operator kept
 // in shared memory
 bool resident_pcg_fits(const LaunchCfg& lc);

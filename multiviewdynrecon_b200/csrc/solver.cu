@@ -280,8 +280,7 @@ static int create_batch(const mvdr_config* cfg, uint32_t B, Batch** out) {
         return fail(MVDR_ECUDA, "cudaFuncSetAttribute failed");
     }
 
-    const uint32_t gmax = std::max<uint32_t>({(lc.max_nodes + 255) / 256, (lc.max_nodes + 31) / 32,
-                                              (lc.max_nodes + 7) / 8, (uint32_t)lc.sm_count * 8}) + 8;
+    const uint32_t gmax = partial_slots(lc);
     // size one instance, then allocate all
     Arena sizing;
     InstDesc tmp{};
