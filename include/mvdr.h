@@ -681,12 +681,16 @@ MVDR_API int mvdr_batch_set_spmv_shape(mvdr_batch* batch, uint32_t shape);
  * captured graphs. MVDR_EINVAL for a matrix-free batch or a batch with more
  * instances than the device holds co-resident CTAs of the kernel. */
 MVDR_API int mvdr_batch_set_pcg_persistent(mvdr_batch* batch, int on);
-/* Bounded waits of the persistent PCG. Each instance barrier gives up after
- * `limit_ns` nanoseconds (default 0.5 s, at most 10 s): the kernel's CTAs
- * return, the instance is flagged and the next checked read reports
- * MVDR_ETIMEOUT; the context stays usable. `extra_arrivals` > 0 makes every
- * barrier wait for that many arrivals beyond the instance's own CTAs, which
- * never come: it exists to exercise the timeout path and is 0 otherwise.
+/* Bounded waits of the PCG forms that run as one cooperative launch: the
+ * persistent PCG, and the resident PCG, which a single mixed-precision
+ * materialised instance of up to 32 nodes per SM runs by default (tile shape 0,
+ * no pcg_tolerance). Each instance barrier gives up after `limit_ns` nanoseconds
+ * (at most 10 s; until set, 0.5 s in the persistent and 2 s in the resident
+ * form): the kernel's CTAs return, the instance is flagged and the next checked
+ * read reports MVDR_ETIMEOUT; the context stays usable. `extra_arrivals` > 0
+ * makes every barrier wait for that many arrivals beyond the instance's own
+ * CTAs, which never come: it exists to exercise the timeout path and is 0
+ * otherwise.
  * The reference has no bounded waits (its PCG is launched kernel by kernel,
  * BlockPCG.cuh:383-458). Drops the captured graphs. */
 MVDR_API int mvdr_batch_set_wait_limit(mvdr_batch* batch, uint64_t limit_ns, uint32_t extra_arrivals);

@@ -2217,9 +2217,6 @@ __global__ void __launch_bounds__(kPersistThreads, 3) pcg_persistent_kernel(cons
 constexpr uint32_t kResidentRows = 32, kResidentTile = 16;   // block rows per CTA and per tile of the SpMV
 constexpr uint32_t kResidentThreads = 12 * kResidentRows;    // 12 threads per block row, as the tile shape
 constexpr uint32_t kResidentEntries = 736;                   // entries kept in shared memory (the others in global memory)
-// every CTA is resident, so a wait ends within microseconds; the limit only
-// keeps a fault elsewhere from hanging the GPU
-constexpr uint64_t kResidentWaitNs = 2000ull * 1000 * 1000;
 constexpr uint32_t kResidentGather = 8;                      // column values per thread loaded before the sums are known
 
 struct ResidentSmem {
@@ -2277,14 +2274,17 @@ __device__ inline bool resident_barrier(const InstDesc& I, ResidentSmem& m, uint
 
 __global__ void __launch_bounds__(kResidentThreads, 1) pcg_resident_kernel(const InstDesc* insts, uint32_t iters,
                                                                            uint32_t nd, uint32_t nq, uint32_t gn,
-                                                                           uint64_t limit_ns) {
+                                                                           uint64_t limit_ns, uint32_t extra) {
     extern __shared__ __align__(16) unsigned char s_resident[];
     ResidentSmem& m = *reinterpret_cast<ResidentSmem*>(s_resident);
     const InstDesc& I = insts[0];
     const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5, G = gridDim.x;
+    const uint32_t arrivals = G + extra;  // of one barrier
     const uint32_t base = blockIdx.x * kResidentRows;
     const uint32_t rows = base < I.N ? min(kResidentRows, I.N - base) : 0u;
     const bool index_ok = index_complete(I);
+    // (a solve that gave up in an earlier iteration does not wait again)
+    if (*(volatile const uint32_t*)&I.counts->error_flags & kErrWaitTimeout) limit_ns = 0;
     // ---- the CTA's rows: entries without the (identity) diagonal
     if (t <= kResidentRows) {
         const uint32_t row = min(base + t, I.N);
@@ -2345,7 +2345,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) pcg_resident_kernel(const
                 I.pcg_hist[(size_t)gn * MVDR_PCG_HISTORY + k] = __longlong_as_double(0x7ff8000000000000ll);
     }
     uint32_t passed = 0;
-    if (!resident_barrier(I, m, ++passed * G, limit_ns)) return;
+    if (!resident_barrier(I, m, ++passed * arrivals, limit_ns)) return;
     // the columns' r^ and d of the first iteration (beta = 0: d = r^)
     for (uint32_t i = t; i < 6 * entries; i += kResidentThreads) {
         const uint32_t e = i / 6, c = i % 6;
@@ -2452,7 +2452,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) pcg_resident_kernel(const
             for (uint32_t w = 0; w < kTileWarps; ++w) sum += m.ws[region][tile * kTileWarps + w];
             I.partials[(size_t)(kRegResident + 3 * parity + region) * I.part_stride + blockIdx.x * kTiles + tile] = sum;
         }
-        if (!resident_barrier(I, m, ++passed * G, limit_ns)) return;
+        if (!resident_barrier(I, m, ++passed * arrivals, limit_ns)) return;
         // ---- the partials' sums (warps 0-3, their loads first) beside the
         // columns' q
         constexpr uint32_t kSteps = 8;
@@ -3108,10 +3108,11 @@ static cudaError_t launch_pcg_persistent(const LaunchCfg& lc, InstDesc* d, uint3
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const uint32_t B = lc.B;
+    const uint64_t limit_ns = lc.wait_limit_ns ? lc.wait_limit_ns : kDefaultWaitLimitNs;
     e = lc.precision == MVDR_PRECISION_MIXED
-            ? cudaLaunchKernelEx(&cfg, pcg_persistent_kernel<true>, (const InstDesc*)d, B, iters, lc.wait_limit_ns,
+            ? cudaLaunchKernelEx(&cfg, pcg_persistent_kernel<true>, (const InstDesc*)d, B, iters, limit_ns,
                                  lc.wait_extra_arrivals)
-            : cudaLaunchKernelEx(&cfg, pcg_persistent_kernel<false>, (const InstDesc*)d, B, iters, lc.wait_limit_ns,
+            : cudaLaunchKernelEx(&cfg, pcg_persistent_kernel<false>, (const InstDesc*)d, B, iters, limit_ns,
                                  lc.wait_extra_arrivals);
     count_launch();
     return e;
@@ -3148,7 +3149,8 @@ static cudaError_t launch_pcg_resident(const LaunchCfg& lc, InstDesc* d, uint32_
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const uint32_t nd = (lc.max_nodes + kPcgNodeThreads - 1) / kPcgNodeThreads;
-    e = cudaLaunchKernelEx(&cfg, pcg_resident_kernel, (const InstDesc*)d, iters, nd, spmv_grid(lc), gn, kResidentWaitNs);
+    e = cudaLaunchKernelEx(&cfg, pcg_resident_kernel, (const InstDesc*)d, iters, nd, spmv_grid(lc), gn,
+                           lc.wait_limit_ns ? lc.wait_limit_ns : kResidentWaitLimitNs, lc.wait_extra_arrivals);
     if (e == cudaSuccess) count_launch();
     return e;
 }

@@ -375,7 +375,7 @@ struct LaunchCfg {
     // bounded waits of the persistent PCG's instance barriers: the limit of
     // each wait, and arrivals each barrier waits for beyond the instance's
     // CTAs (non-zero only to exercise the timeout path)
-    uint64_t wait_limit_ns;
+    uint64_t wait_limit_ns;  // of the PCG barriers (0: the form's default)
     uint32_t wait_extra_arrivals;
     float pcg_tol;  // PCG convergence tolerance (0: fixed iteration count)
     int recompute_jr;  // matrix-free products re-derive the pixel terms' records
@@ -384,7 +384,10 @@ struct LaunchCfg {
 
 constexpr uint32_t kPcgHistRows = 64;  // GN iterations whose PCG residuals are kept
 
-constexpr uint64_t kDefaultWaitLimitNs = 500ull * 1000 * 1000;  // a barrier step takes microseconds
+// limits of the PCG barriers' waits (a step takes microseconds): the persistent
+// form's, and the resident form's, which a caller has not chosen and which
+// therefore bears more
+constexpr uint64_t kDefaultWaitLimitNs = 500ull * 1000 * 1000, kResidentWaitLimitNs = 2000ull * 1000 * 1000;
 constexpr uint64_t kMaxWaitLimitNs = 10ull * 1000 * 1000 * 1000;
 
 // ----------------------------------------------------------- launchers --

@@ -315,7 +315,7 @@ static int create_batch(const mvdr_config* cfg, uint32_t B, Batch** out) {
     }
     b->lc.pcg_bars = b->d_bars;
     b->lc.pcg_persistent = 0;
-    b->lc.wait_limit_ns = kDefaultWaitLimitNs;
+    b->lc.wait_limit_ns = 0;
     b->lc.wait_extra_arrivals = 0;
     b->lc.pcg_grid = persistent_pcg_grid(lc.precision == MVDR_PRECISION_MIXED, lc.sm_count);
     b->owned.resize(B);

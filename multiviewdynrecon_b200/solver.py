@@ -319,7 +319,8 @@ class BatchSolver:
         check(lib().mvdr_batch_set_pcg_persistent(self.h, 1 if on else 0))
 
     def set_wait_limit(self, limit_ns, extra_arrivals=0):
-        """Limit of each bounded barrier wait of the persistent PCG;
+        """Limit of each bounded barrier wait of the persistent and the
+        resident PCG (see mvdr_batch_set_wait_limit);
         extra_arrivals > 0 makes every barrier wait for arrivals that never
         come (exercises the MVDR_ETIMEOUT path)."""
         check(lib().mvdr_batch_set_wait_limit(self.h, int(limit_ns), int(extra_arrivals)))

@@ -100,6 +100,36 @@ def test_persistent_barrier_timeout_is_reported():
     b.close()
 
 
+def test_resident_barrier_timeout_is_reported():
+    """A single instance's PCG (one resident launch by default) gives up at the same
+    limit, and the iterations behind the one that gave up do not wait again."""
+    scene = small_scene("torso")
+    b = BatchSolver(abi.make_config(scene), 1)
+    b.set_input(0, scene)
+    b.solve(2, 5, use_graph=False)
+    want = b.node_se3(0)
+    limit_ms = 40
+    b.set_wait_limit(limit_ms * 1_000_000, extra_arrivals=1)  # one arrival that never comes
+    b.set_input(0, scene)
+    torch.cuda.synchronize()
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    start.record()
+    b.solve(8, 5, use_graph=False)
+    end.record()
+    torch.cuda.synchronize()
+    assert limit_ms < start.elapsed_time(end) < 3 * limit_ms  # (eight waits would be 320 ms)
+    with pytest.raises(MvdrError) as e:
+        b.node_se3(0)
+    assert e.value.status == abi.MVDR_ETIMEOUT
+    # back to a usual limit: the same batch solves cleanly again, also as a graph
+    b.set_wait_limit(500_000_000, extra_arrivals=0)
+    for use_graph in (False, True):
+        b.set_input(0, scene)
+        b.solve(2, 5, use_graph=use_graph)
+        assert torch.equal(b.node_se3(0), want)
+    b.close()
+
+
 def test_wait_limit_arguments_are_checked():
     scene = small_scene("torso")
     b = BatchSolver(abi.make_config(scene), 1)
