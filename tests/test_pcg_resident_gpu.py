@@ -76,3 +76,65 @@ def test_solvers_on_several_streams():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def _rounds(solver, inputs, want, count):
+    """`count` solves on a stream of its own; a failed call raises in the caller."""
+    import torch
+    stream = torch.cuda.Stream()
+    out = torch.empty_like(want).pin_memory()
+    for k in range(count):
+        out.zero_()
+        solver.set_solver_input(inputs, stream=stream)
+        solver.solve_non_rigid_alignment(3, 10, stream=stream)
+        solver.solved_node_se3_async(out, stream=stream)
+        assert solver.counts(stream=stream).error_flags == 0, k
+        assert torch.equal(out, want), k
+    return count
+
+
+def test_launches_that_do_not_fit_together():
+    """Each solver's launch takes most or all of the SMs, so no two of them can be
+    resident at once: the launches take turns, and no barrier waits for the other."""
+    import torch
+    from concurrent.futures import ThreadPoolExecutor
+    from multiviewdynrecon_b200.solver import NonRigidSolver
+    scene, work = _scene(700), []
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for nodes in (4096, 32 * sms, 3000):
+        cfg = abi.make_config(scene, precision=abi.PRECISION_MIXED)
+        cfg.max_nodes, cfg.max_node_pairs = nodes, 16 * nodes
+        g = NonRigidSolver(cfg)
+        inputs = g.set_solver_input(scene)
+        g.solve_non_rigid_alignment(3, 10)
+        work.append((g, inputs, g.solved_node_se3().cpu()))
+    torch.cuda.synchronize()
+    with ThreadPoolExecutor(len(work)) as pool:
+        done = [pool.submit(_rounds, g, inputs, want, 20) for g, inputs, want in work]
+        assert [d.result() for d in done] == [20, 20, 20]
+
+
+def test_one_instance_lanes_as_graphs():
+    """Two lanes of one instance each, whose graphs hold a resident launch per
+    iteration, replayed side by side: the results of single solvers."""
+    import torch
+    from multiviewdynrecon_b200.solver import NonRigidSolver, StreamedBatch
+    scenes = [_scene(700), _scene(600)]
+    cfg = abi.make_config(None, max_nodes=4096, max_views=2, width=96, height=72, use_foreground=True,
+                          use_feature=True, use_cross_view=True, max_surfels=max(s.num_surfels for s in scenes),
+                          max_feature_terms=max(s.feature.count for s in scenes),
+                          max_cross_terms=max(s.cross_view.count for s in scenes))
+    want = []
+    for s in scenes:
+        g = NonRigidSolver(cfg)
+        g.set_solver_input(s)
+        g.solve_non_rigid_alignment(3, 10)
+        want.append(g.solved_node_se3())
+    lanes = StreamedBatch(cfg, 2, lanes=2)
+    for _ in range(20):
+        for i, s in enumerate(scenes):
+            lanes.set_input(i, s)
+        lanes.solve(3, 10)
+        for i in range(2):
+            assert torch.equal(lanes.node_se3(i), want[i])
+    lanes.close()
