@@ -677,7 +677,8 @@ MVDR_API int mvdr_batch_set_spmv_shape(mvdr_batch* batch, uint32_t shape);
 /* on != 0: run each PCG solve of a materialised batch as one persistent
  * cooperative launch (the CTAs split among the instances, each instance's
  * CTAs stepping through its iterations with their own barriers) instead of
- * two or three launches per iteration; on == 0 restores the launches. Drops the
+ * two or three launches per iteration; on == 0 restores the default (those
+ * launches, or the resident PCG of a single instance). Drops the
  * captured graphs. MVDR_EINVAL for a matrix-free batch or a batch with more
  * instances than the device holds co-resident CTAs of the kernel. */
 MVDR_API int mvdr_batch_set_pcg_persistent(mvdr_batch* batch, int on);
@@ -722,7 +723,10 @@ enum {
 /* Enqueue the kernels of one stage for every instance of the batch, with the
  * lambdas of Gauss-Newton iteration 0. The stage reads the state left by the
  * previous solve and overwrites that stage's outputs, so a later solve must
- * start again from mvdr_batch_set_inputs. No host synchronisation. */
+ * start again from mvdr_batch_set_inputs. No host synchronisation. The SpMV, PCG
+ * update and direction stages are the launches of the launched PCG; a solve whose
+ * PCG is one launch (persistent, or resident: see mvdr_batch_set_wait_limit) runs
+ * none of them. */
 MVDR_API int mvdr_batch_enqueue_stage(mvdr_batch* batch, int stage, void* stream);
 
 /* Text of the last error recorded on this host thread. */
