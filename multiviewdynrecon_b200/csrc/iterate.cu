@@ -877,7 +877,9 @@ constexpr uint32_t kPairGroups = kPairChunk / 16;  // groups of 16 lanes per CTA
 template <class Acc>
 __device__ inline void pair_by_thread(const InstDesc& I, const TermOffsets& off, const mvdr_penalty& lam, uint32_t h,
                                       Acc* blocks) {
-    constexpr uint32_t G = sizeof(Acc) == 8 ? 2 : 3;  // (the records in flight fill the registers)
+    // (as many records in flight as the registers of four CTAs per SM hold; with 104
+    // bytes spilled in double, 12 in float)
+    constexpr uint32_t G = sizeof(Acc) == 8 ? 2 : 3;
     const uint32_t Td = off.o[0];
     const bool dens_on = I.use_density && lam.density != 0.f;
     const float4* jr = I.term_jr;
@@ -2211,9 +2213,10 @@ __global__ void __launch_bounds__(kPersistThreads, 3) pcg_persistent_kernel(cons
 // and their order are those of pcg_spmv_scaled_kernel<16, 2, 0> and
 // pcg_update_kernel with their roundings written out, so the increments are the
 // same to the bit.
-// An iteration takes 6.2 us against 13.5 for the two launches with their gaps (4096-node
-// frame; the whole solve 2300 -> 1634 us, a 500-node frame 1445 -> 1225), about half of it
-// the barrier and the partial sums behind it.
+// An iteration took 6.2 us against 13.5 for the two launches with their gaps (4096-node
+// frame; the whole solve 2390 -> 1634 us, a 500-node frame 1480 -> 1225), about half of it
+// the barrier and the partial sums behind it; now 5.5 us (5.0 of 500 nodes), 100 us for
+// 15 iterations (resident_barrier).
 constexpr uint32_t kResidentRows = 32, kResidentTile = 16;   // block rows per CTA and per tile of the SpMV
 constexpr uint32_t kResidentThreads = 12 * kResidentRows;    // 12 threads per block row, as the tile shape
 constexpr uint32_t kResidentEntries = 736;                   // entries kept in shared memory (the others in global memory)
@@ -2390,7 +2393,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) pcg_resident_kernel(const
             }
 #pragma unroll 2
             for (; e < min(e1, kResidentEntries); e += 2) {
-                if (e < u1) break;  // (the lower entries reach past the shared ones)
                 const float2* b2 = reinterpret_cast<const float2*>(&m.blk[e][6 * rr]);
                 const float2* x2 = reinterpret_cast<const float2*>(m.df[kResidentRows + e]);
                 const float2 b01 = b2[0], b23 = b2[1], b45 = b2[2], x01 = x2[0], x23 = x2[1], x45 = x2[2];
@@ -3085,7 +3087,9 @@ uint32_t partial_slots(const LaunchCfg& lc) {
     n = max(n, (lc.max_nodes + 7) / 8);
     n = max(n, (lc.max_nodes + kResidentRows - 1) / kResidentRows * (kResidentRows / kResidentTile));
     for (const SpmvShape& shape : kSpmvShapes) n = max(n, (lc.max_nodes + shape.rows - 1) / shape.rows);
-    return n;
+    // (eight unused ones, for the spacing: a 4,096-node matrix-free solve takes 3053 us
+    // with them, 3060 without)
+    return n + 8;
 }
 
 uint32_t persistent_pcg_grid(int mixed, int sm_count) {
@@ -3294,7 +3298,8 @@ cudaError_t launch_stage(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& l
             else MVDR_LAUNCH((pcg_direction_kernel<false, false>), grid2(gvec, lc.B), 256, 0, st, d, 0, 0, gnode, ~0u, 1u);
             break;
         case MVDR_STAGE_PCG_UPDATE:
-            // (the form the solve runs; no residual history)
+            // (the launched form, no residual history; a resident solve runs neither this
+            // nor the SpMV launch)
             if (scaled) MVDR_LAUNCH((pcg_update_kernel<true, true, true>), grid2(gnode, lc.B), fused_update_threads(lc), 0, st, d, 0, gnode, spmv_grid(lc), ~0u, 1u);
             else if (mixed) MVDR_LAUNCH((pcg_update_kernel<true, false, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, 0, gnode, spmv_grid(lc), ~0u, 1u);
             else MVDR_LAUNCH((pcg_update_kernel<false, false, false>), grid2(gnode, lc.B), kPcgNodeThreads, 0, st, d, 0, gnode, spmv_grid(lc), ~0u, 1u);
