@@ -32,18 +32,15 @@ inline void launch_chained(void (*kernel)(P...), dim3 grid, uint32_t block, size
     count_launch();
 }
 
-// The kernels of a single instance's solve are launched chained, where each
+// The kernels of a solve are launched chained for up to three instances, where each
 // takes 2 to 25 us and the gaps between them count. us, plain / PCG chained / all: a
 // 500-node frame 842 / 842 / 801, 2,048 nodes in FP32 1281 / 1117 / 1063, 4,096 nodes 1566
 // / 1566 / 1463 and matrix-free 3784 / 3370 / 3300, 32,768 nodes 14300 / 13680 / 13700. In
-// batches the waiting blocks hold places that the kernel before them or the other
-// lane's kernels could use: plain / chained, two instances of 4,096 nodes 2175 / 2333,
-// in FP32 of 2,048 1167 / 1198, matrix-free 4614 / 4867, of 500 nodes 822 / 827; three
-// instances 2634 / 2762, 1441 / 1540, 7013 / 7135 and 923 / 923; 16 frames in two lanes
-// 10.17 / 10.26 ms, an uneven batch 7.43 / 7.63 ms. For the same reason the
+// batches the waiting blocks hold places that the other lane's kernels could use: 16
+// frames 10.17 -> 10.26 ms, an uneven batch 7.43 -> 7.63 ms. For the same reason the
 // factorisation, next to which other branches of the assembly run, is launched plainly
 // (chained: 1512 us for 4,096 nodes), as is a kernel that follows a join of streams.
-inline bool chain_kernels(const LaunchCfg& lc) { return lc.B == 1; }
+inline bool chain_kernels(const LaunchCfg& lc) { return lc.B < 4; }
 
 // `chained` (a host value): launch_chained, else MVDR_LAUNCH
 #define MVDR_LAUNCH_IF_CHAINED(chained, kernel, grid, block, smem, stream, ...)            \
