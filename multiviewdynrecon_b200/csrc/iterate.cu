@@ -2997,12 +2997,11 @@ static void launch_diag(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& la
 // 1439 / 1518 / -, 6,000 1957 / 1924 / 1977 / 2080, 9,000 2279 / 2217 / 2188 / 2184, 13,000
 // 2421 / 2347 / 2312 / 2280; larger images, ms, 8,000 11.1 / 11.3 / 13.8 / 16.4, 16,000 12.3
 // / 12.15 / 12.0 / 12.1, 32,768 (128 / 32) 16.2 / 15.8; 16 x 4,096 nodes in two lanes (128 /
-// 32 / 8) 10.74 / 10.53 / 10.31; 2 x 12,000 nodes (32 / 8) 3105 / 3085 us, with larger
-// images 4182 / 4160, 3 x 8,000 3429 / 3400, 3 x 12,000 4406 / 4366.
+// 32 / 8) 10.74 / 10.53 / 10.31.
 static uint32_t group_share(const LaunchCfg& lc) {
     const uint64_t nodes = (uint64_t)lc.B * lc.max_nodes;
     if (nodes < 16384) return nodes < 5120 ? 512 : nodes < 10240 ? 256 : 128;
-    return lc.B == 1 ? 32 : 8;
+    return lc.B < 4 ? 32 : 8;
 }
 // the off-diagonal blocks: the long pairs (by group), the others (by thread)
 template <bool MIXED> static void launch_offdiag_group(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
@@ -3044,9 +3043,7 @@ cudaError_t launch_assemble_forked(const LaunchCfg& lc, InstDesc* d, const mvdr_
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(fork.side[k], fork.begin, 0);
     if (e != cudaSuccess) return e;
     launch_offdiag_thread(lc, d, lam, fork.side[0]);
-    // (a batch fills the GPU: a third branch made 16 x 4096 nodes 1 % slower; two
-    // instances of 4,096 nodes 2229 -> 2173 us with it, three 2719 -> 2638, FP32 of
-    // 2,048 nodes 1311 -> 1167 and 1602 -> 1445)
+    // (a batch fills the GPU: a third branch made 16 x 4096 nodes 1 % slower)
     launch_offdiag_group(lc, d, lam, lc.B < 4 ? fork.side[1] : st);
     launch_diag(lc, d, lam, st);
     // the joins are made even after a failed record, so that a capture ends
@@ -3069,9 +3066,8 @@ cudaError_t launch_energy(const LaunchCfg& lc, InstDesc* d, uint32_t slot, cudaS
 
 // Threads of the fused update: a warp per partial region, or (in batches, whose
 // other instances fill the SMs meanwhile) two warps with two regions each. us:
-// 32,768-node frame 8.3 / 11.7, 4096-node frame 3.4 / 4.0; whole solves of two and three
-// instances of 4,096 nodes 2173 / 2214, 2638 / 2691, of 12,000 3121 / 3234, 4414 / 4509;
-// uneven batch's solve, ms, 8.15 / 8.06.
+// 32,768-node frame 8.3 / 11.7, 4096-node frame 3.4 / 4.0; uneven batch's solve, ms,
+// 8.15 / 8.06.
 static uint32_t fused_update_threads(const LaunchCfg& lc) { return kPcgNodeThreads * (lc.B < 4 ? 2 : 1); }
 
 // CTAs per instance of the SpMV launch with the current shape
