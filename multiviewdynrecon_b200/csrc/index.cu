@@ -796,9 +796,9 @@ __global__ void __launch_bounds__(32 * kRowWarps) np_row_count_kernel(const Inst
 // ranked, which gives each one's start; a second pass places the entries: of 32
 // consecutive terms, those of the same partner take consecutive places in lane
 // order. Both passes take kRowSlices slices of 32 terms at once, so that their
-// gathers overlap; bound by those gathers and by fetching its own unrolled
-// instructions: with four slices (80 registers) 32,768 nodes take 929 us and 500
-// nodes the same 101, with one 580 and 118. A term that lists a partner twice, or a
+// gathers overlap; bound by those gathers and by the table's traffic in shared memory
+// (32,768 nodes: that pipe 58 % busy, a third of the warps): with four slices (80
+// registers) 32,768 nodes take 929 us and 500 nodes the same 101, with one 580 and 118. A term that lists a partner twice, or a
 // node with more than kRowPartners partners, takes the sweep (one pass over the
 // list per partner), which is what every node took before: 285 -> 101 us on a
 // 500-node frame, whose lists reach 1,276 terms (54 with a CTA per node), 72 -> 51 us

@@ -813,8 +813,8 @@ __device__ inline void twist_row(Acc px, Acc py, Acc pz, uint32_t c, Acc (&g)[6]
 // same order with the same operations and give the same bits.
 // The longer of the two launches, us, against one thread per pair with one
 // record in flight: 500-node frame 62 (was 262), 2048-node FP32 frame 63 (308),
-// 4096-node frame 70 (197), 32,768-node frame 317 (663; half of its record
-// gathers miss the L2).
+// 4096-node frame 70 (197), 32,768-node frame 317 (663; 56 % of its L2 reads
+// go on to DRAM).
 
 // the pair's smooth terms' points (p_i, p_j), has[m]: the term is valid
 template <class Acc>
@@ -2997,7 +2997,9 @@ static void launch_diag(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& la
 // 1439 / 1518 / -, 6,000 1957 / 1924 / 1977 / 2080, 9,000 2279 / 2217 / 2188 / 2184, 13,000
 // 2421 / 2347 / 2312 / 2280; larger images, ms, 8,000 11.1 / 11.3 / 13.8 / 16.4, 16,000 12.3
 // / 12.15 / 12.0 / 12.1, 32,768 (128 / 32) 16.2 / 15.8; 16 x 4,096 nodes in two lanes (128 /
-// 32 / 8) 10.74 / 10.53 / 10.31.
+// 32 / 8) 10.74 / 10.53 / 10.31; two and three instances (32 / 8), us, 2 x 12,000 nodes
+// 3229 / 3203, 3 x 12,000 4547 / 4509, 2 x 9,000 with larger images on a stream 4335 /
+// 4458.
 static uint32_t group_share(const LaunchCfg& lc) {
     const uint64_t nodes = (uint64_t)lc.B * lc.max_nodes;
     if (nodes < 16384) return nodes < 5120 ? 512 : nodes < 10240 ? 256 : 128;
@@ -3043,7 +3045,9 @@ cudaError_t launch_assemble_forked(const LaunchCfg& lc, InstDesc* d, const mvdr_
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(fork.side[k], fork.begin, 0);
     if (e != cudaSuccess) return e;
     launch_offdiag_thread(lc, d, lam, fork.side[0]);
-    // (a batch fills the GPU: a third branch made 16 x 4096 nodes 1 % slower)
+    // (a batch fills the GPU: a third branch made 16 x 4096 nodes 1 % slower; two
+    // instances of 4,096 nodes 2388 -> 2333 us with it, three 2842 -> 2762, FP32 of
+    // 2,048 nodes 1343 -> 1198 and 1696 -> 1540)
     launch_offdiag_group(lc, d, lam, lc.B < 4 ? fork.side[1] : st);
     launch_diag(lc, d, lam, st);
     // the joins are made even after a failed record, so that a capture ends
@@ -3066,8 +3070,9 @@ cudaError_t launch_energy(const LaunchCfg& lc, InstDesc* d, uint32_t slot, cudaS
 
 // Threads of the fused update: a warp per partial region, or (in batches, whose
 // other instances fill the SMs meanwhile) two warps with two regions each. us:
-// 32,768-node frame 8.3 / 11.7, 4096-node frame 3.4 / 4.0; uneven batch's solve, ms,
-// 8.15 / 8.06.
+// 32,768-node frame 8.3 / 11.7, 4096-node frame 3.4 / 4.0; whole solves of two and three
+// instances of 4,096 nodes 2333 / 2422, 2762 / 2983; uneven batch's solve, ms, 8.15 /
+// 8.06.
 static uint32_t fused_update_threads(const LaunchCfg& lc) { return kPcgNodeThreads * (lc.B < 4 ? 2 : 1); }
 
 // CTAs per instance of the SpMV launch with the current shape
@@ -3083,9 +3088,9 @@ uint32_t partial_slots(const LaunchCfg& lc) {
     n = max(n, (lc.max_nodes + 7) / 8);
     n = max(n, (lc.max_nodes + kResidentRows - 1) / kResidentRows * (kResidentRows / kResidentTile));
     for (const SpmvShape& shape : kSpmvShapes) n = max(n, (lc.max_nodes + shape.rows - 1) / shape.rows);
-    // (eight unused ones, for the spacing: a 4,096-node matrix-free solve takes 3053 us
-    // with them, 3060 without)
-    return n + 8;
+    // (regions on lines of their own: a 32,768-node frame 13.67 ms, with 8,200 slots
+    // 13.73, a 19,860-node frame 2797 us, with 4,973 slots 2823)
+    return (n / 32 + 1) * 32;
 }
 
 uint32_t persistent_pcg_grid(int mixed, int sm_count) {
