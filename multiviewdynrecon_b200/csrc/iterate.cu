@@ -2609,7 +2609,7 @@ __device__ inline void load_node6(int fused, const Acc* dv, const float* xin, ui
 // are one Jacobian row scaled by each node's skinning weight, so its J.p is
 // that row times the weight-blended p (one record load per term). With
 // `fused` set p is the PCG direction d of this iteration, else xin.
-template <bool MIXED, bool RECOMP>
+template <bool MIXED, bool RECOMP, bool PIXELS_LAST>
 __global__ void __launch_bounds__(256, RECOMP ? 2 : 4) apply_j_kernel(const InstDesc* insts, const float* xin, int parity, int fused,
                                                       mvdr_penalty lam) {
     chain_wait();
@@ -2623,10 +2623,8 @@ __global__ void __launch_bounds__(256, RECOMP ? 2 : 4) apply_j_kernel(const Inst
     // mixed precision keeps J.p in double (jp holds 3 doubles per term)
     Acc* jp = reinterpret_cast<Acc*>(I.jp);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < T; i += gridDim.x * blockDim.x) {
-        // The terms that are no pixels take longest (a chain of loads per node): they
-        // go first, not at the end of the last wave, which makes a 4,096-node
-        // matrix-free frame 3290 -> 3093 us.
-        const uint32_t t = i < T - off.o[0] ? i + off.o[0] : i - (T - off.o[0]);
+        uint32_t t = i;
+        if constexpr (PIXELS_LAST) t = i < T - off.o[0] ? i + off.o[0] : i - (T - off.o[0]);
         uint32_t k;
         const TermType ty = off.typed(t, k);
         const ushort4 nn = term_nodes(I, ty, k);
@@ -2955,6 +2953,23 @@ static uint32_t scale_grid(const LaunchCfg& lc) {
     return min((lc.cap_pairs + kScalePairsPerCta - 1) / kScalePairsPerCta, (uint32_t)lc.sm_count * 16);
 }
 
+// The terms that are no pixels take longest (a chain of loads per node). First instead
+// of at the end of the last wave they shorten a small launch; a large one has other
+// work to run beside them and loses the order of its reads (apply_j_kernel's
+// PIXELS_LAST). Whole matrix-free solves, us, pixels first / last: 1, 2, 4 instances of
+// 1,500 nodes 3780 / 3660, 5755 / 5680, 9578 / 9520, of 4,096 3157 / 2980, 4952 / 4840, 9420 /
+// 9383; 1, 2, 4 of 12,000 4165 / 4160, 7037 / 7177, 13290 / 13400; one of 20,000 with larger
+// images 16885 / 16990; 8 and 16 of 1,500 16276 / 16356, 29208 / 29488, of 4,096 17310 /
+// 17455, 32530 / 33213.
+static int pixels_last(const LaunchCfg& lc) { return lc.B <= 4 && (uint64_t)lc.B * lc.max_nodes <= 16384; }
+
+template <bool MIXED, bool RECOMP>
+static void launch_apply_j(const LaunchCfg& lc, InstDesc* d, const float* x, int parity, int fused, uint32_t gterm,
+                           uint32_t B, const mvdr_penalty& lam, cudaStream_t st) {
+    auto* kernel = pixels_last(lc) ? &apply_j_kernel<MIXED, RECOMP, true> : &apply_j_kernel<MIXED, RECOMP, false>;
+    MVDR_LAUNCH_IF_CHAINED(fused && chain_kernels(lc), kernel, grid2(gterm, B), 256, 0, st, d, x, parity, fused, lam);
+}
+
 // J.d then Jt.(J.d) (+ damping): `fused` takes the PCG direction of `parity`
 // as the operand and stores q with its d.q partials, else x -> y
 static void launch_apply_pair(const LaunchCfg& lc, InstDesc* d, const float* x, float* y, int parity, int fused,
@@ -2962,16 +2977,16 @@ static void launch_apply_pair(const LaunchCfg& lc, InstDesc* d, const float* x, 
     const bool chain = fused && chain_kernels(lc);
     const bool mixed = lc.precision == MVDR_PRECISION_MIXED;
     if (mixed && lc.recompute_jr) {
-        MVDR_LAUNCH_IF_CHAINED(chain, (apply_j_kernel<true, true>), grid2(gterm, B), 256, 0, st, d, x, parity, fused, lam);
+        launch_apply_j<true, true>(lc, d, x, parity, fused, gterm, B, lam, st);
         MVDR_LAUNCH_IF_CHAINED(chain, (apply_jt_kernel<true, true>), grid2(gwarp, B), 256, 0, st, d, x, y, fused, parity, lam);
     } else if (mixed) {
-        MVDR_LAUNCH_IF_CHAINED(chain, (apply_j_kernel<true, false>), grid2(gterm, B), 256, 0, st, d, x, parity, fused, lam);
+        launch_apply_j<true, false>(lc, d, x, parity, fused, gterm, B, lam, st);
         MVDR_LAUNCH_IF_CHAINED(chain, (apply_jt_kernel<true, false>), grid2(gwarp, B), 256, 0, st, d, x, y, fused, parity, lam);
     } else if (lc.recompute_jr) {
-        MVDR_LAUNCH_IF_CHAINED(chain, (apply_j_kernel<false, true>), grid2(gterm, B), 256, 0, st, d, x, parity, fused, lam);
+        launch_apply_j<false, true>(lc, d, x, parity, fused, gterm, B, lam, st);
         MVDR_LAUNCH_IF_CHAINED(chain, (apply_jt_kernel<false, true>), grid2(gwarp, B), 256, 0, st, d, x, y, fused, parity, lam);
     } else {
-        MVDR_LAUNCH_IF_CHAINED(chain, (apply_j_kernel<false, false>), grid2(gterm, B), 256, 0, st, d, x, parity, fused, lam);
+        launch_apply_j<false, false>(lc, d, x, parity, fused, gterm, B, lam, st);
         MVDR_LAUNCH_IF_CHAINED(chain, (apply_jt_kernel<false, false>), grid2(gwarp, B), 256, 0, st, d, x, y, fused, parity, lam);
     }
 }
