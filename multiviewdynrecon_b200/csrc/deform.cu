@@ -375,9 +375,16 @@ __device__ inline unsigned long long to_fixed(float v) {
 // are integers: exact, whatever the order. A value below 2^50 is added as two limbs
 // of 25 bits, because a node may be all four of a surfel's (a scene of one node) and
 // so be added 32 x 4 times; a warp with a larger or negative value adds pixel by
-// pixel. Five views of 1280 x 720, 32,768 nodes: 364 -> 282 us, of which the issue
-// slots and the L1 are busy a good half each (59 registers: 44 % of the warps).
+// pixel, as does one with many nodes. Five views of 1280 x 720, 32,768 nodes: 364 -> 282 -> 279 us, of
+// which the issue slots and the L1 are busy a good half each (59 registers: 44 % of
+// the warps).
 constexpr uint32_t kTileX = 32, kTileY = 8;  // pixels of a CTA
+// A tile whose pixels have more nearest nodes than this is added pixel by pixel: each
+// node of a summed tile costs a round, and few entries share it. us, atomics per pixel /
+// tile sums / this: three views of 640 x 480, 32,768 nodes 37.3 / 41.5 / 36.2, 8,000 nodes
+// 40.5 / 35.4 / 34.8, five of 1280 x 720 close by 369 / 277 / 275 (limits of 4, 8, 12, 16: 35.8,
+// 37.0, 38.8, 40.3; 34.5, 35.1, 35.7, 35.9; 275, 278, 279, 279).
+constexpr uint32_t kTileNodes = 6;
 constexpr uint32_t kLimbBits = 25, kLimbMask = (1u << kLimbBits) - 1u;
 static_assert(32ull * 4 * kLimbMask <= 0xFFFFFFFFull, "a warp's sum of one limb fits 32 bits");
 
@@ -408,7 +415,8 @@ __global__ void __launch_bounds__(256) node_error_kernel(const InstDesc* __restr
         }
         all |= es[k] | ws[k];
     }
-    if (__any_sync(0xffffffffu, (all >> (2 * kLimbBits)) != 0)) {
+    const uint32_t nearest = __popc(__ballot_sync(0xffffffffu, lane + 1 == __ffs(__match_any_sync(0xffffffffu, nk[0]))));
+    if (nearest > kTileNodes || __any_sync(0xffffffffu, (all >> (2 * kLimbBits)) != 0)) {
         if (err > 1e-6f) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
