@@ -3034,8 +3034,24 @@ static void launch_offdiag_group(const LaunchCfg& lc, InstDesc* d, const mvdr_pe
 static void launch_offdiag_thread(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {
     const uint32_t share = group_share(lc);
     const dim3 grid = grid2(min(pair_slots(lc.cap_pairs) / kPairChunk, (uint32_t)lc.sm_count * 16), lc.B);
-    if (lc.precision == MVDR_PRECISION_MIXED) MVDR_LAUNCH(offdiag_thread_kernel<true>, grid, kPairChunk, 0, st, d, lam, share);
-    else MVDR_LAUNCH(offdiag_thread_kernel<false>, grid, kPairChunk, 0, st, d, lam, share);
+    // With the density term a pair's entries gather two records each, and the neighbours'
+    // gathers hit in the L1. Beside the diagonal or the group kernel, which set up much
+    // of it as shared memory, the launch took three times as long, depending on which of
+    // the three reached an SM first: an FP32 frame of 15,043 nodes 3630 or 4570 us from one
+    // solver to the next. So it asks for SMs that are set up as L1: 3610 each time.
+    // (Without the term it is left to mix: 4,096 nodes 1320 us, 1353 with the request.)
+    cudaLaunchAttribute l1;
+    l1.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    l1.val.sharedMemCarveout = cudaSharedmemCarveoutMaxL1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kPairChunk);
+    cfg.stream = st;
+    cfg.attrs = &l1;
+    cfg.numAttrs = lc.use_density ? 1 : 0;
+    auto* kernel = lc.precision == MVDR_PRECISION_MIXED ? &offdiag_thread_kernel<true> : &offdiag_thread_kernel<false>;
+    cudaLaunchKernelEx(&cfg, kernel, (const InstDesc*)d, lam, share);
+    count_launch();
 }
 
 cudaError_t launch_assemble(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, bool materialize,
