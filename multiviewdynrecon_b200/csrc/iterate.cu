@@ -3015,8 +3015,15 @@ static void launch_diag(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& la
 // 32 / 8) 10.74 / 10.53 / 10.31; two and three instances (32 / 8), us, 2 x 12,000 nodes
 // 3229 / 3203, 3 x 12,000 4547 / 4509, 2 x 9,000 with larger images on a stream 4335 /
 // 4458.
+// A batch whose images have less than 100 pixels a node has short lists, so that the few
+// are enough from 5,120 nodes on (batches in two lanes, by the shares for their nodes /
+// 8; one thread per pair): 12 x 1,700 2268 / 2152 (2235), 12 x 2,080 2504 / 2425 (2417), 16 x
+// 1,000 1982 / 1899 (1994), 8 x 3,000 2632 / 2545 (2632), 8 x 1,300 at 107 pixels 1659 /
+// 1627 (1849); with sizes from half of 2,000 up, at 460 pixels, 2950 / 3243 (4387).
 static uint32_t group_share(const LaunchCfg& lc) {
     const uint64_t nodes = (uint64_t)lc.B * lc.max_nodes;
+    const uint64_t pixels = (uint64_t)lc.max_views * lc.width * lc.height;
+    if (lc.B >= 4 && nodes >= 5120 && pixels < 100ull * lc.max_nodes) return 8;
     if (nodes < 16384) return nodes < 5120 ? 512 : nodes < 10240 ? 256 : 128;
     return lc.B < 4 ? 32 : 8;
 }

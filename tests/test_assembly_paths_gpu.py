@@ -96,3 +96,28 @@ def test_blocks_do_not_depend_on_the_share_taken_by_group():
         solver.close()
     for blocks in got[1:]:
         assert np.array_equal(blocks, got[0])
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_MIXED, abi.PRECISION_FP32])
+@pytest.mark.parametrize("count,capacity", [(4, 1279), (4, 1280), (5, 1300), (4, 4096)])
+def test_batches_at_each_share_of_pairs(precision, count, capacity):
+    """A batch with little image per node takes fewer pairs by group from 5,120 nodes of
+    capacity on: the bits of a single solve on both sides of the line."""
+    import torch
+    from multiviewdynrecon_b200.solver import BatchSolver, NonRigidSolver
+    scene = synth.sphere_single_view(seed=3, num_nodes=300, width=160, height=120)
+    cfg = abi.make_config(scene, precision=precision)
+    single = NonRigidSolver(cfg)
+    single.set_solver_input(scene)
+    single.solve_non_rigid_alignment(2, 6)
+    want = single.get_array(abi.ARRAY_INCREMENT)
+    cfg.max_nodes, cfg.max_node_pairs = capacity, 32 * scene.num_nodes
+    b = BatchSolver(cfg, count)
+    for i in range(count):
+        b.set_input(i, scene)
+    b.solve(2, 6)
+    torch.cuda.synchronize()
+    for i in range(count):
+        assert np.array_equal(b.instance(i).get_array(abi.ARRAY_INCREMENT), want)
+    b.close()
+    single.close()
