@@ -32,21 +32,21 @@ inline void launch_chained(void (*kernel)(P...), dim3 grid, uint32_t block, size
     count_launch();
 }
 
-// The kernels of a solve are launched chained for up to three instances, where each
-// takes 2 to 25 us and the gaps between them count. us, plain / PCG chained / all: a
-// 500-node frame 842 / 842 / 801, 2,048 nodes in FP32 1281 / 1117 / 1063, 4,096 nodes 1566
-// / 1566 / 1463 and matrix-free 3784 / 3370 / 3300, 32,768 nodes 14300 / 13680 / 13700. Two
-// and three instances, plain / chained: enqueued on a stream, 1,200 nodes 2616 / 2151 and
-// 3093 / 2629, 4,096 nodes 2724 / 2422 and 3135 / 2857, matrix-free 5287 / 4906 and 7855 /
-// 7372; replayed as a graph, 1,200 nodes 2162 / 2131 and 2561 / 2514, 4,096 nodes 2272 /
-// 2332 and 2699 / 2752, in FP32 2239 / 2497 and 2711 / 2898, matrix-free 4565 / 4801 and 7087
-// / 7245. In lanes the waiting blocks hold places that the other lane's kernels could
-// use: two lanes of two of 1,200 nodes 2890 / 3111, of three 3711 / 3944 (the launch does
-// not know of other lanes), 16 frames 10.17 / 10.26 ms, an uneven batch 7.43 / 7.63 ms.
-// For the same reason the factorisation, next to which other branches of the assembly
-// run, is launched plainly (chained: 1512 us for 4,096 nodes), as is a kernel that
-// follows a join of streams.
-inline bool chain_kernels(const LaunchCfg& lc) { return lc.B < 4; }
+// The kernels of a solve of up to three instances are launched chained where the call
+// enqueues them on a stream (LaunchCfg::chained): each takes 2 to 25 us, and the gaps
+// between them count. us, plain / PCG chained / all: a 500-node frame 842 / 842 / 801,
+// 2,048 nodes in FP32 1281 / 1117 / 1063, 4,096 nodes 1566 / 1566 / 1463 and matrix-free 3784
+// / 3370 / 3300, 32,768 nodes 14300 / 13680 / 13700; plain / chained, two and three
+// instances of 1,200 nodes 2616 / 2151 and 3093 / 2629, of 4,096 2724 / 2422 and 3135 /
+// 2857. Plainly in the graphs that a batch captures, where the gaps are shorter and
+// other lanes' kernels could use the places that waiting blocks hold: two lanes of two
+// instances of 1,200 nodes 2890 / 3111, of 4,096 3305 / 3497, of three 3711 / 3944 and 4520 /
+// 4637; 16 frames 10.17 / 10.26 ms, an uneven batch 7.43 / 7.63 ms; one lane of one, two
+// and three instances of 4,096 nodes 1388 / 1395, 2272 / 2332 and 2699 / 2752, a 32,768-node
+// frame 13240 / 13370, but 2,000 nodes in FP32 1788 / 1687. For the same reason the
+// factorisation, next to which other branches of the assembly run, is launched plainly
+// (chained: 1512 us for 4,096 nodes), as is a kernel that follows a join of streams.
+inline bool chain_kernels(const LaunchCfg& lc) { return lc.chained != 0; }
 
 // `chained` (a host value): launch_chained, else MVDR_LAUNCH
 #define MVDR_LAUNCH_IF_CHAINED(chained, kernel, grid, block, smem, stream, ...)            \

@@ -380,6 +380,7 @@ struct LaunchCfg {
     float pcg_tol;  // PCG convergence tolerance (0: fixed iteration count)
     int recompute_jr;  // matrix-free products re-derive the pixel terms' records
     int resident;      // the PCG may run as one resident launch (resident_pcg_fits)
+    int chained;       // the kernels are launched chained (chain_kernels)
 };
 
 constexpr uint32_t kPcgHistRows = 64;  // GN iterations whose PCG residuals are kept

@@ -269,6 +269,7 @@ static int create_batch(const mvdr_config* cfg, uint32_t B, Batch** out) {
     lc.recompute_jr = cfg->recompute_jacobians ? 1 : 0;
     lc.sm_count = prop.multiProcessorCount;
     lc.resident = resident_pcg_fits(lc) ? 1 : 0;
+    lc.chained = B < 4 ? 1 : 0;
 
     const size_t smem_seg = (size_t)lc.cap_seg * 4;
     if (smem_seg > (size_t)prop.sharedMemPerBlockOptin) {
@@ -644,40 +645,40 @@ struct NvtxRange {
     ~NvtxRange() { nvtxRangePop(); }
 };
 
-static int enqueue_index(Batch& b, cudaStream_t st) {
+static int enqueue_index(Batch& b, const LaunchCfg& lc, cudaStream_t st) {
     NvtxRange range("mvdr/index");
     // zero the per-build counters of every instance
     for (uint32_t i = 0; i < b.B; ++i) {
         const InstDesc& I = b.host[i];
         CU(cudaMemsetAsync(I.counts, 0, sizeof(DeviceCounts), st));
-        CU(cudaMemsetAsync(I.n2t_count, 0, sizeof(uint32_t) * (b.lc.max_nodes + 1), st));
+        CU(cudaMemsetAsync(I.n2t_count, 0, sizeof(uint32_t) * (lc.max_nodes + 1), st));
     }
-    CU(launch_build_index(b.lc, b.d_inst, st));
+    CU(launch_build_index(lc, b.d_inst, st));
     return MVDR_OK;
 }
 
-static int enqueue_iteration(Batch& b, uint32_t iter, uint32_t pcg, cudaStream_t st) {
+static int enqueue_iteration(Batch& b, const LaunchCfg& lc, uint32_t iter, uint32_t pcg, cudaStream_t st) {
     NvtxRange range("mvdr/gn_iteration");
     const mvdr_penalty lam = penalty_for(b.cfg, iter);
     {
         NvtxRange r("mvdr/terms");
-        CU(launch_eval_terms(b.lc, b.d_inst, lam, st));
-        CU(launch_energy(b.lc, b.d_inst, std::min<uint32_t>(iter, 63), st));
+        CU(launch_eval_terms(lc, b.d_inst, lam, st));
+        CU(launch_energy(lc, b.d_inst, std::min<uint32_t>(iter, 63), st));
     }
     {
         NvtxRange r("mvdr/assemble");
         if (b.cfg.mode == MVDR_MODE_MATERIALIZED)
-            CU(launch_assemble_forked(b.lc, b.d_inst, lam, st, b.fork));
+            CU(launch_assemble_forked(lc, b.d_inst, lam, st, b.fork));
         else
-            CU(launch_assemble(b.lc, b.d_inst, lam, false, st));
+            CU(launch_assemble(lc, b.d_inst, lam, false, st));
     }
     {
         NvtxRange r("mvdr/pcg");
-        CU(launch_pcg(b.lc, b.d_inst, lam, pcg, iter, st));
+        CU(launch_pcg(lc, b.d_inst, lam, pcg, iter, st));
     }
     {
         NvtxRange r("mvdr/update");
-        CU(launch_update(b.lc, b.d_inst, st));
+        CU(launch_update(lc, b.d_inst, st));
     }
     return MVDR_OK;
 }
@@ -688,10 +689,10 @@ static int solve_batch(Batch& b, uint32_t gn, uint32_t pcg, bool graph, cudaStre
     if (rc != MVDR_OK) return rc;
     if (gn > 63) return fail(MVDR_EINVAL, "at most 63 Gauss-Newton iterations per solve");
     if (!graph) {
-        rc = enqueue_index(b, st);
+        rc = enqueue_index(b, b.lc, st);
         if (rc != MVDR_OK) return rc;
         for (uint32_t k = 0; k < gn; ++k) {
-            rc = enqueue_iteration(b, k, pcg, st);
+            rc = enqueue_iteration(b, b.lc, k, pcg, st);
             if (rc != MVDR_OK) return rc;
         }
         b.gn_iter = gn;
@@ -710,8 +711,10 @@ static int solve_batch(Batch& b, uint32_t gn, uint32_t pcg, bool graph, cudaStre
             cudaStreamDestroy(cap);
             return fail(MVDR_ECUDA, std::string("begin capture: ") + cudaGetErrorString(e));
         }
-        rc = enqueue_index(b, cap);
-        for (uint32_t k = 0; rc == MVDR_OK && k < gn; ++k) rc = enqueue_iteration(b, k, pcg, cap);
+        LaunchCfg lc = b.lc;
+        lc.chained = 0;
+        rc = enqueue_index(b, lc, cap);
+        for (uint32_t k = 0; rc == MVDR_OK && k < gn; ++k) rc = enqueue_iteration(b, lc, k, pcg, cap);
         e = cudaStreamEndCapture(cap, &g);
         cudaStreamDestroy(cap);
         if (rc != MVDR_OK) {
@@ -917,7 +920,7 @@ int mvdr_build_index(mvdr_solver* s, void* stream) {
     if (!s->owns) return fail(MVDR_EINVAL, "use mvdr_batch_solve for batch members");
     int rc = all_bound(*s->batch);
     if (rc != MVDR_OK) return rc;
-    rc = enqueue_index(*s->batch, (cudaStream_t)stream);
+    rc = enqueue_index(*s->batch, s->batch->lc, (cudaStream_t)stream);
     if (rc == MVDR_OK) s->batch->gn_iter = 0;
     return rc;
 }
@@ -929,7 +932,7 @@ int mvdr_gn_iteration(mvdr_solver* s, uint32_t pcg_iterations, void* stream) {
     int rc = all_bound(b);
     if (rc != MVDR_OK) return rc;
     if (b.gn_iter >= 63) return fail(MVDR_EINVAL, "too many Gauss-Newton iterations");
-    rc = enqueue_iteration(b, b.gn_iter, pcg_iterations, (cudaStream_t)stream);
+    rc = enqueue_iteration(b, b.lc, b.gn_iter, pcg_iterations, (cudaStream_t)stream);
     if (rc == MVDR_OK) b.gn_iter++;
     return rc;
 }
@@ -1044,8 +1047,8 @@ int mvdr_batch_autotune(mvdr_batch* bh, void* stream, double* times_ms, uint32_t
     if (b.cfg.mode == MVDR_MODE_MATERIALIZED) {
         int rc = all_bound(b);
         if (rc != MVDR_OK) return rc;
-        rc = enqueue_index(b, st);
-        if (rc == MVDR_OK) rc = enqueue_iteration(b, 0, 1, st);
+        rc = enqueue_index(b, b.lc, st);
+        if (rc == MVDR_OK) rc = enqueue_iteration(b, b.lc, 0, 1, st);
         if (rc != MVDR_OK) return rc;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         CU(cudaEventCreate(&e0));
@@ -1129,7 +1132,7 @@ int mvdr_batch_enqueue_stage(mvdr_batch* b, int stage, void* stream) {
     Batch& bb = *b->batch;
     int rc = all_bound(bb);
     if (rc != MVDR_OK) return rc;
-    if (stage == MVDR_STAGE_INDEX) return enqueue_index(bb, (cudaStream_t)stream);
+    if (stage == MVDR_STAGE_INDEX) return enqueue_index(bb, bb.lc, (cudaStream_t)stream);
     if (stage < MVDR_STAGE_INDEX || stage > MVDR_STAGE_SCALE) return fail(MVDR_EINVAL, "unknown stage");
     // the J.d scratch exists only in the matrix-free mode
     if (stage == MVDR_STAGE_MATRIX_FREE && bb.cfg.mode != MVDR_MODE_MATRIX_FREE)

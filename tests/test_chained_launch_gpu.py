@@ -6,7 +6,7 @@ import torch
 
 from conftest import small_scene
 from multiviewdynrecon_b200 import abi
-from multiviewdynrecon_b200.solver import NonRigidSolver
+from multiviewdynrecon_b200.solver import BatchSolver, NonRigidSolver
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,24 @@ def test_captured_iterations_equal_plain_ones(precision, mode):
     assert np.array_equal(solver.get_array(abi.ARRAY_INCREMENT), want[0])
     assert np.array_equal(solver.get_array(abi.ARRAY_NODE_SE3), want[1])
     solver.close()
+
+
+@pytest.mark.parametrize("precision,mode", [(abi.PRECISION_FP32, abi.MODE_MATERIALIZED),
+                                            (abi.PRECISION_MIXED, abi.MODE_MATERIALIZED),
+                                            (abi.PRECISION_MIXED, abi.MODE_MATRIX_FREE)])
+@pytest.mark.parametrize("count", [1, 2, 3, 4])
+def test_chained_streams_equal_plain_graphs(precision, mode, count):
+    """Up to three instances are launched chained on a stream and plainly in the batch's
+    graph: the same bits."""
+    scene = small_scene("torso")
+    b = BatchSolver(abi.make_config(scene, precision=precision, mode=mode), count)
+    got = []
+    for use_graph in (False, True, True, False):
+        for i in range(count):
+            b.set_input(i, scene)
+        b.solve(3, 7, use_graph=use_graph)
+        torch.cuda.synchronize()
+        got.append([b.instance(i).get_array(abi.ARRAY_NODE_SE3) for i in range(count)])
+    for x in got:
+        assert all(np.array_equal(a, got[0][0]) for a in x)
+    b.close()
