@@ -3015,17 +3015,19 @@ static void launch_diag(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& la
 // 32 / 8) 10.74 / 10.53 / 10.31; two and three instances (32 / 8), us, 2 x 12,000 nodes
 // 3229 / 3203, 3 x 12,000 4547 / 4509, 2 x 9,000 with larger images on a stream 4335 /
 // 4458.
-// A batch whose images have less than 100 pixels a node has short lists, so that the few
-// are enough from 5,120 nodes on (batches in two lanes, by the shares for their nodes /
-// 8; one thread per pair): 12 x 1,700 2268 / 2152 (2235), 12 x 2,080 2504 / 2425 (2417), 16 x
+// A batch has its other instances' chains to fill the GPU: the few from 12,288 nodes on,
+// and from 5,120 where the images have less than 100 pixels a node and the lists are
+// short. Batches in two lanes, by a single instance's shares / 8 (one thread per pair):
+// 8 x 3,500 nodes of two views of 640 x 480 3471 / 3344 (3641), 11 x up to 1,738 at 116
+// pixels 2214 / 2256 (2745), 12 x 1,700 2268 / 2152 (2235), 12 x 2,080 2504 / 2425 (2417), 16 x
 // 1,000 1982 / 1899 (1994), 8 x 3,000 2632 / 2545 (2632), 8 x 1,300 at 107 pixels 1659 /
 // 1627 (1849); with sizes from half of 2,000 up, at 460 pixels, 2950 / 3243 (4387).
 static uint32_t group_share(const LaunchCfg& lc) {
     const uint64_t nodes = (uint64_t)lc.B * lc.max_nodes;
     const uint64_t pixels = (uint64_t)lc.max_views * lc.width * lc.height;
-    if (lc.B >= 4 && nodes >= 5120 && pixels < 100ull * lc.max_nodes) return 8;
+    if (lc.B >= 4 && (nodes >= 12288 || (nodes >= 5120 && pixels < 100ull * lc.max_nodes))) return 8;
     if (nodes < 16384) return nodes < 5120 ? 512 : nodes < 10240 ? 256 : 128;
-    return lc.B < 4 ? 32 : 8;
+    return 32;
 }
 // the off-diagonal blocks: the long pairs (by group), the others (by thread)
 template <bool MIXED> static void launch_offdiag_group(const LaunchCfg& lc, InstDesc* d, const mvdr_penalty& lam, cudaStream_t st) {

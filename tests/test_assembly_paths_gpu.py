@@ -99,7 +99,7 @@ def test_blocks_do_not_depend_on_the_share_taken_by_group():
 
 
 @pytest.mark.parametrize("precision", [abi.PRECISION_MIXED, abi.PRECISION_FP32])
-@pytest.mark.parametrize("count,capacity", [(4, 1279), (4, 1280), (5, 1300), (4, 4096)])
+@pytest.mark.parametrize("count,capacity", [(4, 1279), (4, 1280), (5, 1300), (4, 3071), (4, 3072)])
 def test_batches_at_each_share_of_pairs(precision, count, capacity):
     """A batch with little image per node takes fewer pairs by group from 5,120 nodes of
     capacity on: the bits of a single solve on both sides of the line."""
