@@ -6,7 +6,7 @@ import torch
 
 from conftest import small_scene
 from multiviewdynrecon_b200 import abi
-from multiviewdynrecon_b200.solver import BatchSolver, NonRigidSolver
+from multiviewdynrecon_b200.solver import NonRigidSolver
 
 pytestmark = pytest.mark.gpu
 
@@ -47,6 +47,7 @@ def test_captured_iterations_equal_plain_ones(precision, mode):
 def test_chained_streams_equal_plain_graphs(precision, mode, count):
     """Up to three instances are launched chained on a stream and plainly in the batch's
     graph: the same bits."""
+    from multiviewdynrecon_b200.solver import BatchSolver
     scene = small_scene("torso")
     b = BatchSolver(abi.make_config(scene, precision=precision, mode=mode), count)
     got = []
